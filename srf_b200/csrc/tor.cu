@@ -24,6 +24,7 @@
 #include <atomic>
 #include <cmath>
 #include <cstdlib>
+#include <cstring>
 #include <type_traits>
 
 #include "lor_prep.cuh"
@@ -34,14 +35,65 @@ namespace {
 
 enum TorOp { kProj = 0, kBack = 1, kMap = 2, kAdj = 3, kCount = 4 };
 
-// Process-wide tuning (srf_tor_set_tuning): kernel family (0 auto, 1 slab with a lane per
-// segment, 2 LOR-centric, 3 slab with items spread over lanes),
+// Process-wide tuning (srf_tor_set_tuning): kernel family (0 auto, 1 and 3 slab with a lane
+// per segment, 2 LOR-centric),
 // slices per slab (0 = as many as fit), grid multiplier of the persistent slab kernel
 // (CTAs = SMs x mult, one resident per SM: more, smaller shares of the segment list;
 // 0 = automatic, see slab_grid_mult).
 std::atomic<int> g_tune_path{0};
 std::atomic<int> g_tune_nsl{0};
 std::atomic<int> g_tune_mult{0};
+
+// ---------------------------------------------------------------------------------
+// Two floats per instruction: sm_100's paired FP32 arithmetic, each half rounded as the
+// scalar operation. Kernels that are bound by instruction issue get two voxel slots of
+// every step of d^2 and of the exponent for one issue slot.
+struct F2 {
+    unsigned long long v;
+};
+// Both halves the same, as kernel parameters (they stay in constant memory, where a pair
+// made in the kernel would take two moves at each use).
+struct PairConsts {
+    F2 ix, iy, lb, bb;  // inter_x, inter_y, l_bound, b_bound
+    F2 one;
+    F2 col[8];          // column centres c + 0.5
+};
+__device__ __forceinline__ F2 pack2(float lo, float hi) {
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ F2 both(float a) { return pack2(a, a); }
+__device__ __forceinline__ void unpack2(F2 p, float &lo, float &hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(p.v));
+}
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+__device__ __forceinline__ F2 mul2(F2 a, F2 b) {
+    F2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+
+__device__ __forceinline__ F2 add2(F2 a, F2 b) {
+    F2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+
+__device__ __forceinline__ F2 sub2(F2 a, F2 b) {
+    F2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 neg2(F2 a) {
+    float lo, hi;
+    unpack2(a, lo, hi);
+    return pack2(-lo, -hi);
+}
 
 struct TorParams {
     const float *x1, *y1, *z1, *x2, *y2, *z2, *xc, *yc, *zc, *f;
@@ -64,7 +116,9 @@ struct TorParams {
     float *proj_out;
     int *count_out;   // kCount: [n] voxels with non-zero weight, [n] window voxels visited
     int use_slab;     // scatter ops: shared-memory slab kernel (1) or global atomics (0)
-    int slab_expand;  // slab kernel: spread items over lanes (1) or a lane per segment (0)
+    float box_x0, box_y0;  // -bound / inter - 1/2: voxel-centre units of a coordinate 0
+    PairConsts pc;    // the geometry as operands of the paired arithmetic (slab kernels)
+    float fit;        // largest box half-extent that no window clips (box_in_window)
     // Batched frames: LOR i belongs to frame frame[i] (null: one frame) whose image starts
     // frame_stride floats after the previous frame's.
     const int *frame;
@@ -474,11 +528,20 @@ __device__ __forceinline__ bool lor_geometry(const TorParams &p, int64_t t, LorC
     }
     const float zlo = fminf(z1, z2), zhi = fmaxf(z1, z2);
     if (!(L.dz != 0.0f && zlo == zlo && zhi == zhi && fabsf(zhi - zlo) <= 3.0e38f)) return false;
-    const float flo = floorf((zlo - p.slice0_f) / p.inter_z) - 2.0f;
-    const float fhi = ceilf((zhi - p.slice0_f) / p.inter_z) + 2.0f;
-    L.s_lo = (int)fmaxf(flo, 0.0f);
-    L.s_hi = (int)fminf(fhi, (float)(p.gz - 1));
+    // every slice the exact test can pass, with a margin far above the rounding here
+    const float flo = (zlo - p.slice0_f) / p.inter_z, fhi = (zhi - p.slice0_f) / p.inter_z;
+    const float margin = 0.01f + 4.0e-6f * fmaxf(fabsf(flo), fabsf(fhi));
+    L.s_lo = (int)fmaxf(ceilf(flo - margin), 0.0f);
+    L.s_hi = (int)fminf(floorf(fhi + margin), (float)(p.gz - 1));
     return L.s_lo <= L.s_hi;
+}
+
+// log2 |v|: |v| = m 2^e with m in [0.5, 1), log2 m from the hardware approximation
+// (absolute error ~2^-22) plus e exactly.
+__device__ __forceinline__ float log2_abs(float v) {
+    int e;
+    const float m = frexpf(fabsf(v), &e);
+    return (float)e + __log2f(m);
 }
 
 // The op's per-LOR output scale from its value (back-projection: tof_scale / v, dropped
@@ -492,11 +555,8 @@ __device__ __forceinline__ bool lor_value_scale(const TorParams &p, int64_t t, L
         if (!((double)v > 1e-7)) return false;  // tor.cu.cc:203
         L.scale = __fdiv_rn(p.tof_scale, v);
         // w * scale = 2^(log2 w + log2 scale): the scale joins the exponent (one add per
-        // slice instead of one multiply per voxel). scale = m 2^e with m in [0.5, 1):
-        // log2 m from the hardware approximation (absolute error ~2^-22) plus e exactly.
-        int e;
-        const float m = frexpf(L.scale, &e);
-        L.k0s = (float)e + __log2f(m);
+        // slice instead of one multiply per voxel)
+        L.k0s = log2_abs(L.scale);
     } else if (OP == kMap) {
         L.scale = __fdiv_rn(1.0f, map_value(p, t));  // tor.cu.cc:239, no threshold
         L.all = !(fabsf(L.scale) <= 3.0e38f);  // w/0 or w/NaN lands on every visited voxel
@@ -535,18 +595,46 @@ __device__ __forceinline__ bool prepare_any(const TorParams &p, int64_t t, LorCo
 // The binning pass stores each LOR's geometry once as a 64-byte record, so the slab
 // kernels take it with four 16-byte loads per segment instead of re-deriving it from the
 // ten columns in every slab the LOR meets:
-//   {x1, y1, z1, d0}, {d1, dz, ux, uy}, {cut, k1, bxv, byv}, {xc, yc, zc, slices}
-// with slices = s_lo | s_hi << 16, or -1 when the LOR contributes nothing.
+//   {x1, y1, z1, d0}, {d1, dz, ux, uy}, {cut, k1, bxv, byv}, {z0, kA, kE, slices}
+// with slices = s_lo | s_hi << 15, bit 30 set for a LOR that takes the general walk.
+//
+// TOF. With X(s) the LOR's point in slice plane z_s, |C - X(s)|^2 is a parabola in z_s:
+// A (z_s - z0)^2 + E, A = 1 + (d0/dz)^2 + (d1/dz)^2, whose vertex z0 is zc up to rounding
+// when C lies on the LOR. The record holds z0 and the two log2 coefficients kA = -a_coef A,
+// kE = -a_coef E, taken in double once per LOR, so a slice's TOF exponent costs a
+// subtraction, a product and an FMA instead of three differences and a dot product.
+//
+// General walk: LORs at more than ~83 degrees from the slice axis (A > kMaxSlope2; a
+// dominant-axis group's have A <= 3), where the vertex form loses digits and few slices
+// are crossed anyway.
 struct __align__(16) LorRec {
     float4 a, b, c, d;
 };
 
-__device__ __forceinline__ LorRec make_rec(const LorConst &L, bool ok) {
+constexpr double kMaxSlope2 = 64.0;
+constexpr int kSliceBits = 15;
+constexpr int kSliceMask = (1 << kSliceBits) - 1;
+
+__device__ __forceinline__ LorRec make_rec(const TorParams &p, const LorConst &L, bool tof) {
+    const double mx = (double)L.d0 / (double)L.dz, my = (double)L.d1 / (double)L.dz;
+    const double A = 1.0 + mx * mx + my * my;
+    float z0 = 0.0f, kA = 0.0f, kE = 0.0f;
+    if (tof) {
+        const double h = (double)L.zc - (double)L.z1;
+        const double ex = (double)L.xc - ((double)L.x1 + mx * h);
+        const double ey = (double)L.yc - ((double)L.y1 + my * h);
+        const double h0 = (ex * mx + ey * my) / A;
+        z0 = (float)((double)L.zc + h0);
+        kA = (float)(-(double)p.a_coef * A);
+        kE = (float)(-(double)p.a_coef * (ex * ex + ey * ey - A * h0 * h0));
+    }
+    const int general = A <= kMaxSlope2 ? 0 : 1 << (2 * kSliceBits);
     LorRec r;
     r.a = make_float4(L.x1, L.y1, L.z1, L.d0);
     r.b = make_float4(L.d1, L.dz, L.ux, L.uy);
     r.c = make_float4(L.cut, L.k1, L.bxv, L.byv);
-    r.d = make_float4(L.xc, L.yc, L.zc, __int_as_float(ok ? (L.s_lo | (L.s_hi << 16)) : -1));
+    r.d = make_float4(z0, kA, kE,
+                      __int_as_float(L.s_lo | (L.s_hi << kSliceBits) | general));
     return r;
 }
 
@@ -558,30 +646,47 @@ __device__ __forceinline__ float4 ldg_f4(const float4 *q) {
     return v;
 }
 
-// LOR t's geometry from its record; false when the LOR contributes nothing.
-__device__ __forceinline__ bool lor_rec_geometry(const LorRec *rec, int64_t t, LorConst &L) {
+// A segment's LOR in the slab kernels, from its record.
+struct SegLor {
+    float x1, y1, z1, d0, d1, dz, inv_dz, ux, uy;
+    float cut, k1, bxv, byv;
+    float z0, kA, kE;
+    float scale;  // per-LOR factor of its weights (back-projection: in kE instead)
+    int s_lo, s_hi;
+    bool general;  // takes general_segment
+};
+
+__device__ __forceinline__ void seg_lor(const LorRec *rec, int64_t t, SegLor &L) {
     const float4 *q = reinterpret_cast<const float4 *>(rec + t);
-    const float4 d = ldg_f4(q + 3);
-    const int sl = __float_as_int(d.w);
-    const float4 a = ldg_f4(q), b = ldg_f4(q + 1), c = ldg_f4(q + 2);
+    const float4 a = ldg_f4(q), b = ldg_f4(q + 1), c = ldg_f4(q + 2), d = ldg_f4(q + 3);
     L.x1 = a.x; L.y1 = a.y; L.z1 = a.z; L.d0 = a.w;
     L.d1 = b.x; L.dz = b.y; L.ux = b.z; L.uy = b.w;
     L.cut = c.x; L.k1 = c.y; L.bxv = c.z; L.byv = c.w;
-    L.xc = d.x; L.yc = d.y; L.zc = d.z;
-    L.s_lo = sl & 0xffff;
-    L.s_hi = sl >> 16;
-    L.all = false;
-    L.k0s = 0.0f;
-    return sl >= 0;
+    L.z0 = d.x; L.kA = d.y; L.kE = d.z;
+    const int sl = __float_as_int(d.w);
+    L.s_lo = sl & kSliceMask;
+    L.s_hi = (sl >> kSliceBits) & kSliceMask;
+    L.general = (sl >> (2 * kSliceBits)) != 0;
+    L.inv_dz = __frcp_rn(L.dz);
 }
 
-// LOR t's constants from its record and the op's value (lor_prepare's result).
+// The op's factor of LOR t's weights (lor_value_scale) in L: a scatter op's magnitude as
+// log2 in kE and by itself in L.scale with its sign, the projection's in L.scale. False
+// when the LOR contributes nothing.
 template <int OP>
-__device__ __forceinline__ bool lor_load(const TorParams &p, const LorRec *rec, int64_t t,
-                                         LorConst &L) {
-    L.scale = p.tof_scale;
-    if (!lor_rec_geometry(rec, t, L)) return false;
-    return lor_value_scale<OP>(p, t, L);
+__device__ __forceinline__ bool seg_value(const TorParams &p, int64_t t, SegLor &L) {
+    LorConst c;
+    c.scale = p.tof_scale;
+    c.k0s = 0.0f;
+    c.all = false;
+    if (!lor_value_scale<OP>(p, t, c)) return false;
+    L.scale = c.scale;
+    L.general = L.general || c.all || !(fabsf(c.scale) <= 3.0e38f);
+    if (OP != kProj) {
+        if (!(fabsf(c.scale) > 0.0f)) return L.general && c.scale != 0.0f;  // 0 adds nothing
+        L.kE += OP == kBack ? c.k0s : log2_abs(c.scale);
+    }
+    return true;
 }
 
 // (int)(a / b) with a correctly rounded quotient, as the reference truncates it
@@ -596,30 +701,17 @@ __device__ __forceinline__ int trunc_div(float a, float b, float inv_b) {
 
 // One voxel slot: the reference's d^2 (tor.cu.cc:61-66, FMA-contracted as nvcc builds
 // it) and cut-off decision, and the folded exponent.
-// `cut` and `all` are the LOR's (L.cut, L.all) for a row the caller walks, -inf and false
-// for a row it must leave out (so the row costs no branch).
 template <int OP, typename F>
-__device__ __forceinline__ void slot(const LorConst &L, float cut, bool all, float dx, float dyuy,
-                                     float dy2, float k0, int ix, int iy, F &f) {
+__device__ __forceinline__ void slot(const LorConst &L, float dx, float dyuy, float dy2,
+                                     float k0, int ix, int iy, F &f) {
     const float rc = __fmaf_rn(dx, L.ux, dyuy);
     const float d2 = __fmaf_rn(-rc, rc, __fmaf_rn(dx, dx, dy2));
-    const bool in_cut = d2 < cut;
+    const bool in_cut = d2 < L.cut;
     const float e = fast_exp2(fmaf(d2, L.k1, k0));
     if (OP == kMap)
-        f(ix, iy, in_cut ? e : 0.0f, in_cut || all);
+        f(ix, iy, in_cut ? e : 0.0f, in_cut || L.all);
     else
         f(ix, iy, e, in_cut);
-}
-
-// W consecutive slots of one row.
-template <int OP, int W, int P, typename F>
-__device__ __forceinline__ void row_slots(const LorConst &L, float cut, bool all,
-                                          const float (&dxs)[P], float dy, float k0, int xlo,
-                                          int iy, F &f) {
-    const float dyuy = __fmul_rn(dy, L.uy);
-    const float dy2 = __fmul_rn(dy, dy);
-#pragma unroll
-    for (int i = 0; i < W; i++) slot<OP>(L, cut, all, dxs[i], dyuy, dy2, k0, xlo + i, iy, f);
 }
 
 // g(std::integral_constant<int, w>{}) for a runtime width 1 <= w <= P.
@@ -635,20 +727,13 @@ __device__ __forceinline__ void with_width(int w, G &&g) {
 }
 
 // One (LOR, slice): the reference's crossing test and window (tor.cu.cc:22-48,
-// :135-136), then the voxels of the window's part inside the tube's bounding box:
+// :135-136), then the voxels of the window's part inside the tube's bounding box, clipped
+// to the grid and to rows R0 <= iy < R1:
 // f(ix, iy, w, use) with w the unscaled weight and use the reference's decision (d^2
 // below the cut-off; for a map LOR with L.all set, every in-slice window voxel, with
 // w = 0 outside the cut-off, as the reference adds 0/0 there). Returns the number of
 // in-slice window voxels (for kCount).
-//
-// Only rows R0 <= iy < R1 are walked (a band of rows of the grid, or all of it).
-// kPadded: the caller's slice has P - 1 zero columns on both sides of the grid and P - 1
-// spare rows above and below the band (the shared-memory slab), so window columns
-// outside the grid need no test: a gather reads 0 there and a scatter lands in padding
-// that is never flushed. The walked box is then widened to the warp's largest (kept
-// inside the window), which makes the trip counts warp-uniform; rows the widening adds
-// outside the band are masked. Otherwise the box is clipped to the grid.
-template <int OP, int P, bool kPadded, bool kBand, typename F>
+template <int OP, int P, typename F>
 __device__ __forceinline__ int slice_visit(const TorParams &p, const LorConst &L, int s, int R0,
                                            int R1, F &&f) {
     const float sz = slice_z<OP>(p, s);
@@ -668,30 +753,12 @@ __device__ __forceinline__ int slice_visit(const TorParams &p, const LorConst &L
     }
     // Bounding box in voxel-centre units (column i has its centre at i + 0.5 voxels).
     const float fx = __fmaf_rn(rx, p.inv_x, -0.5f), fy = __fmaf_rn(ry, p.inv_y, -0.5f);
-    int xlo = max(ix0, __float2int_ru(fx - L.bxv));
-    int xhi = min(ix0 + P - 1, __float2int_rd(fx + L.bxv));
-    int ylo = max(iy0, __float2int_ru(fy - L.byv));
-    int yhi = min(iy0 + P - 1, __float2int_rd(fy + L.byv));
-    // A slab holding whole slices has zero padding rows too; only a band needs row limits.
-    constexpr bool banded = !kPadded || kBand;
-    if (banded) {
-        ylo = max(ylo, R0);
-        yhi = min(yhi, R1 - 1);
-    }
-    if (!kPadded) {
-        xlo = max(xlo, 0);
-        xhi = min(xhi, p.gx - 1);
-    }
-    int wx = xhi - xlo + 1, wy = yhi - ylo + 1;
+    const int xlo = max(max(ix0, __float2int_ru(fx - L.bxv)), 0);
+    const int xhi = min(min(ix0 + P - 1, __float2int_rd(fx + L.bxv)), p.gx - 1);
+    const int ylo = max(max(iy0, __float2int_ru(fy - L.byv)), R0);
+    const int yhi = min(min(iy0 + P - 1, __float2int_rd(fy + L.byv)), R1 - 1);
+    const int wx = xhi - xlo + 1, wy = yhi - ylo + 1;
     if (wx <= 0 || wy <= 0) return n_slots;
-    if (kPadded) {
-        const unsigned am = __activemask();
-        const int mx = __reduce_max_sync(am, wx), my = __reduce_max_sync(am, wy);
-        xlo = min(xlo, ix0 + P - mx);  // still inside the window, still covers the box
-        ylo = min(ylo, iy0 + P - my);
-        wx = mx;
-        wy = my;
-    }
     float k0 = OP == kBack ? L.k0s : 0.0f;
     if (OP != kMap && OP != kCount && p.tof_on) {
         const float ax = __fsub_rn(L.xc, cx), ay = __fsub_rn(L.yc, cy), az = __fsub_rn(L.zc, sz);
@@ -705,66 +772,17 @@ __device__ __forceinline__ int slice_visit(const TorParams &p, const LorConst &L
         const float mxi = __fmaf_rn(p.inter_x, fx0 + ((float)i + 0.5f), p.l_bound);
         dxs[i] = __fsub_rn(cx, mxi);
     }
-    if (kPadded) {
-        // wx, wy are warp-uniform: one fully unrolled row body per width, so that a row's
-        // loads issue back to back. The gather picks the body once per slice; the scatter
-        // (a compare-and-swap loop per voxel in shared memory) runs faster picking it per
-        // row (measured).
-        // In a band, rows the widening added outside [R0, R1) (another band's, or off
-        // the grid) are masked through their cut-off; the walked rows stay within the
-        // slab's padding rows. Whole slices need no mask (their padding rows read 0).
-        const float fy0 = (float)ylo + 0.5f;
-        auto walk = [&](auto masked) {
-            constexpr bool kMask = decltype(masked)::value;
-            auto row_cut = [&](int j, bool &all) {
-                if constexpr (kMask) {
-                    const bool in_band = (unsigned)(ylo + j - R0) < (unsigned)(R1 - R0);
-                    all = in_band && L.all;
-                    return in_band ? L.cut : -INFINITY;
-                } else {
-                    all = L.all;
-                    return L.cut;
-                }
-            };
-            // fj = ylo + j + 0.5 (a half-integer: adding 1 per row is exact)
-            if (OP == kProj) {
-                with_width<P>(wx, [&](auto W) {
-                    float fj = fy0;
-                    for (int j = 0; j < wy; j++, fj += 1.0f) {
-                        bool all;
-                        const float cut = row_cut(j, all);
-                        const float dy = __fsub_rn(cy, __fmaf_rn(p.inter_y, fj, p.b_bound));
-                        row_slots<OP, decltype(W)::value>(L, cut, all, dxs, dy, k0, xlo, ylo + j,
-                                                          f);
-                    }
-                });
-            } else {
-                float fj = fy0;
-                for (int j = 0; j < wy; j++, fj += 1.0f) {
-                    bool all;
-                    const float cut = row_cut(j, all);
-                    const float dy = __fsub_rn(cy, __fmaf_rn(p.inter_y, fj, p.b_bound));
-                    with_width<P>(wx, [&](auto W) {
-                        row_slots<OP, decltype(W)::value>(L, cut, all, dxs, dy, k0, xlo, ylo + j,
-                                                          f);
-                    });
-                }
-            }
-        };
-        walk(std::integral_constant<bool, kBand>{});
-    } else {
 #pragma unroll
-        for (int j = 0; j < P; j++) {
-            if (j >= wy) break;
-            const int iy = ylo + j;
-            const float dy = __fsub_rn(cy, __fmaf_rn(p.inter_y, (float)iy + 0.5f, p.b_bound));
-            const float dyuy = __fmul_rn(dy, L.uy);
-            const float dy2 = __fmul_rn(dy, dy);
+    for (int j = 0; j < P; j++) {
+        if (j >= wy) break;
+        const int iy = ylo + j;
+        const float dy = __fsub_rn(cy, __fmaf_rn(p.inter_y, (float)iy + 0.5f, p.b_bound));
+        const float dyuy = __fmul_rn(dy, L.uy);
+        const float dy2 = __fmul_rn(dy, dy);
 #pragma unroll
-            for (int i = 0; i < P; i++) {
-                if (i >= wx) break;
-                slot<OP>(L, L.cut, L.all, dxs[i], dyuy, dy2, k0, xlo + i, iy, f);
-            }
+        for (int i = 0; i < P; i++) {
+            if (i >= wx) break;
+            slot<OP>(L, dxs[i], dyuy, dy2, k0, xlo + i, iy, f);
         }
     }
     return n_slots;
@@ -786,7 +804,7 @@ __global__ void __launch_bounds__(256) tor_kernel_p(const TorParams p) {
             const int64_t img0 = frame_offset(p, t);
             for (int s = L.s_lo + lane; s <= L.s_hi; s += 32) {
                 const int64_t base = img0 + (int64_t)s * p.sz;
-                n_slots += slice_visit<OP, P, false, false>(p, L, s, 0, p.gy,
+                n_slots += slice_visit<OP, P>(p, L, s, 0, p.gy,
                                                      [&](int ix, int iy, float w, bool use) {
                     const int64_t idx = base + (int64_t)iy * p.sy + (int64_t)ix * p.sx;
                     if (OP == kCount) {
@@ -839,8 +857,13 @@ constexpr int kSegThreads = 512;
 constexpr int kSegItems = 8;
 constexpr int kSegTile = kSegThreads * kSegItems;
 constexpr int kMaxSlabs = 4096;
-constexpr int kSlabThreads = 1024;
+constexpr int kProjThreads = 896;
+constexpr int kScatThreads = 1024;
+// Threads of a slab CTA (one CTA per SM).
+constexpr int slab_threads(int op) { return op == kProj ? kProjThreads : kScatThreads; }
 constexpr size_t kSlabSmemBytes = 220 * 1024;  // of the 227 KB a CTA can opt into
+constexpr int kMaxSlabSlices = 1024;           // entries of the slab's table of slice planes
+constexpr size_t kSlabSmemMax = kSlabSmemBytes + sizeof(float) * kMaxSlabSlices;
 // Budget of the per-slab LOR lists of one chunk of LORs (srf_tor_set_scratch_limit). The
 // lists are sized for the worst case (every slab of a frame), so the budget sets how many
 // chunks a call over row-band slabs takes, each a full pass (slab loads and flushes again):
@@ -1013,7 +1036,7 @@ __global__ void __launch_bounds__(kSegThreads) seg_count_kernel(const TorParams 
         if (t < p.n) {
             ok = geometry_any<OP>(p, t, L);  // generated map LORs are made here
             if (ok) {  // only LORs that enter the slab lists are ever read back
-                const LorRec r = make_rec(L, ok);
+                const LorRec r = make_rec(p, L, OP != kMap && p.tof_on);
                 float4 *q = reinterpret_cast<float4 *>(sp.rec + t);
                 q[0] = r.a;
                 q[1] = r.b;
@@ -1118,8 +1141,8 @@ __global__ void __launch_bounds__(kSegThreads) seg_fill_kernel(const TorParams p
             const float4 *q = reinterpret_cast<const float4 *>(sp.rec + t);
             const float4 a = q[0], b = q[1], d = q[3];
             const int sl = __float_as_int(d.w);
-            s_lo = sl & 0xffff;
-            s_hi = sl >> 16;
+            s_lo = sl & kSliceMask;
+            s_hi = (sl >> kSliceBits) & kSliceMask;
             y1 = a.y;
             z1 = a.z;
             d1 = b.x;
@@ -1153,31 +1176,255 @@ __host__ __device__ __forceinline__ int slab_floats(int nsl, int gx, int gy, int
     return nsl * slab_slice_stride(gx, gy, pad) + slab_origin(gx, pad);
 }
 
+// a / b correctly rounded, given inv_b = 1 / b correctly rounded: the quotient estimate
+// a * inv_b and one step with its exact remainder (P. Markstein, "Computation of elementary
+// functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990). Equal to the
+// division on 6e8 random and boundary arguments of the ranges that occur here (results
+// below 2^-126 excepted, which no decision here depends on).
+__device__ __forceinline__ float div_by(float a, float b, float inv_b) {
+    const float q = __fmul_rn(a, inv_b);
+    return __fmaf_rn(__fmaf_rn(-q, b, a), inv_b, q);
+}
+
+// Where a slab sits and how its shared memory is laid out.
+struct SlabView {
+    float *mem;       // the slab's words
+    const float *zs;  // plane of each of its slices
+    int rs, ss;       // row and slice stride
+    unsigned base;    // word of (slice 0, row 0 of the grid, column 0), less kMagicBits (rs + 1)
+    int R0, R1;       // rows of the grid it covers
+};
+
+// Adding 1.5 * 2^23 to a float below 2^22 in magnitude leaves its integer part (rounded as
+// the add is told to) in the low bits: floor and ceiling without a conversion.
+constexpr float kMagic = 12582912.0f;
+constexpr unsigned kMagicBits = 0x4B400000u;
+
+// One slice of a segment: where its box starts and the terms its voxels share.
+struct SliceBox {
+    float cx, cy;  // crossing point
+    float xm, ym;  // first column and row of the box, as kMagic + integer
+    float k0;      // exponent at d^2 = 0
+    bool in;
+};
+
+// The crossing (tor.cu.cc:22-48) of slice s (counted from the slab's first) and the first
+// column and row of the H x W box that is walked there.
+//
+// kWindow: the reference's window (tor.cu.cc:135-136) is the box (W = H = P). Without, the box
+// starts at the first voxel centre within the half-extents of the crossing: only for LORs
+// whose half-extents are below TorParams::fit, of which the window clips no voxel wherever
+// they cross, so it decides nothing (every LOR of a dominant-axis group, up to rounding,
+// where the voxels are cubes: the patch is made for extents up to sqrt 2 times the radius).
+template <int OP, int P, int W, bool kWindow>
+__device__ __forceinline__ SliceBox slice_box(const TorParams &p, const SlabView &v,
+                                              const SegLor &L, int s, bool valid, float lo_x,
+                                              float lo_y, int H) {
+    SliceBox b;
+    const float sz = v.zs[valid ? s : 0];
+    const float ratio = div_by(__fsub_rn(sz, L.z1), L.dz, L.inv_dz);
+    b.cx = __fmaf_rn(L.d0, ratio, L.x1);
+    b.cy = __fmaf_rn(L.d1, ratio, L.y1);
+    if (kWindow) {
+        b.xm = truncf(div_by(__fsub_rn(b.cx, p.l_bound), p.inter_x, p.inv_x)) +
+               (kMagic - (float)p.half);
+        b.ym = truncf(div_by(__fsub_rn(b.cy, p.b_bound), p.inter_y, p.inv_y)) +
+               (kMagic - (float)p.half);
+    } else {
+        b.xm = __fadd_ru(fmaf(b.cx, p.inv_x, lo_x), kMagic);
+        b.ym = __fadd_ru(fmaf(b.cy, p.inv_y, lo_y), kMagic);
+    }
+    b.in = valid && ratio > 0.0f && ratio < 1.0f && b.xm > kMagic - (float)W &&
+           b.xm < kMagic + (float)p.gx && b.ym > kMagic + (float)(v.R0 - H) &&
+           b.ym < kMagic + (float)v.R1;
+    b.k0 = L.kE;
+    if (OP != kMap && p.tof_on) {
+        const float h = sz - L.z0;
+        b.k0 = fmaf(h * h, L.kA, L.kE);
+    }
+    return b;
+}
+
+// The slices a .. a + cnt - 1 (counted from the slab's first) of the lane's segment; the
+// warp's lanes walk n_max slices together, H rows and W columns of each (at least every
+// lane's own box). Projection: returns the sum of w * slab. Scatter ops: adds the weights.
+//
+// These kernels are bound by instruction issue and FP32 throughput (the earlier form issued
+// on 86 % of the cycles): of ~420 lane-instructions per (LOR, slice) only ~125 were the
+// voxels, the rest set-up. Here the set-up has no division, no conversion and one branch:
+// the crossing's quotient comes from a reciprocal (div_by), the box's start from an add
+// that rounds up, the plane from a table, the box's size is fixed per segment (a box of
+// half-extent b holds at most floor(2 b) + 1 voxel centres) instead of reduced over the warp
+// in every slice, and the window is left out where it decides nothing. Two slices go side
+// by side through columns, rows and voxels, two floats per instruction (halving the loops'
+// own cost; one slice at a time measured 5.25 ms against 5.07 for the projection of 10M
+// events); a slice that is not crossed follows its
+// neighbour with a cut-off nothing passes. Rows outside the slab's rows lie in its padding,
+// which reads 0 and is never flushed.
+template <int OP, int P, int W, bool kWindow>
+__device__ __forceinline__ float walk_segment(const TorParams &p, const SlabView &v,
+                                              const SegLor &L, int a, int cnt, int n_max,
+                                              int H) {
+    const float lo_x = p.box_x0 - L.bxv, lo_y = p.box_y0 - L.byv;
+    const F2 ux2 = both(L.ux), uy2 = both(L.uy), k1 = both(L.k1);
+    float acc0 = 0.0f, acc1 = 0.0f;
+    for (int i = 0; i < n_max; i += 2) {
+        const SliceBox b0 = slice_box<OP, P, W, kWindow>(p, v, L, a + i, i < cnt, lo_x, lo_y, H);
+        const SliceBox b1 = slice_box<OP, P, W, kWindow>(p, v, L, a + i + 1, i + 1 < cnt, lo_x,
+                                                         lo_y, H);
+        if (b0.in || b1.in) {
+            unsigned o0 = __float_as_uint(b0.ym) * (unsigned)v.rs + __float_as_uint(b0.xm) +
+                          (unsigned)((a + i) * v.ss) + v.base;
+            unsigned o1 = __float_as_uint(b1.ym) * (unsigned)v.rs + __float_as_uint(b1.xm) +
+                          (unsigned)((a + i + 1) * v.ss) + v.base;
+            if (!b0.in) o0 = o1;
+            if (!b1.in) o1 = o0;
+            const float n0 = b0.in ? L.cut : -INFINITY, n1 = b1.in ? L.cut : -INFINITY;
+            float *r0 = v.mem + (int)o0, *r1 = v.mem + (int)o1;
+            const F2 k0 = pack2(b0.k0, b1.k0);
+            F2 dx[W];
+            {
+                const F2 cx = pack2(b0.cx, b1.cx), xl = pack2(b0.xm - kMagic, b1.xm - kMagic);
+#pragma unroll
+                for (int c = 0; c < W; c++)
+                    dx[c] = sub2(cx, fma2(p.pc.ix, add2(xl, p.pc.col[c]), p.pc.lb));
+            }
+            const F2 cy = pack2(b0.cy, b1.cy);
+            F2 yc = pack2((b0.ym - kMagic) + 0.5f, (b1.ym - kMagic) + 0.5f);  // exact
+#pragma unroll 1
+            for (int j = 0; j < H; j++) {
+                const F2 dy = sub2(cy, fma2(p.pc.iy, yc, p.pc.bb));
+                const F2 dyuy = mul2(dy, uy2), dy2 = mul2(dy, dy);
+#pragma unroll
+                for (int c = 0; c < W; c++) {
+                    // tor.cu.cc:61-66, FMA-contracted as nvcc builds it
+                    const F2 rc = fma2(dx[c], ux2, dyuy);
+                    const F2 d2 = fma2(neg2(rc), rc, fma2(dx[c], dx[c], dy2));
+                    const F2 ex = fma2(d2, k1, k0);
+                    float d0, d1, e0, e1;
+                    unpack2(d2, d0, d1);
+                    unpack2(ex, e0, e1);
+                    const float w0 = fast_exp2(e0), w1 = fast_exp2(e1);
+                    if (OP == kProj) {
+                        if (d0 < n0) acc0 = fmaf(w0, r0[c], acc0);
+                        if (d1 < n1) acc1 = fmaf(w1, r1[c], acc1);
+                    } else {
+                        if (d0 < n0) atomicAdd(r0 + c, L.scale < 0.0f ? -w0 : w0);
+                        if (d1 < n1) atomicAdd(r1 + c, L.scale < 0.0f ? -w1 : w1);
+                    }
+                }
+                r0 += v.rs;
+                r1 += v.rs;
+                yc = add2(yc, p.pc.one);
+            }
+        }
+        __syncwarp();
+    }
+    return acc0 + acc1;
+}
+
+// A segment whose LOR takes the general walk (a map LOR with a zero or non-finite divisor,
+// a LOR far from the slice axis): its slices [S0, S1) and rows [R0, R1) straight on the
+// image in global memory.
+template <int OP, int P>
+__device__ __noinline__ void general_segment(const TorParams &p, int64_t t, int S0, int S1,
+                                             int R0, int R1, int64_t img0) {
+    LorConst L;
+    if (!prepare_any<OP>(p, t, L)) return;
+    float acc = 0.0f;
+    for (int s = max(L.s_lo, S0); s <= min(L.s_hi, S1 - 1); s++) {
+        const int64_t base = img0 + (int64_t)s * p.sz;
+        slice_visit<OP, P>(p, L, s, R0, R1, [&](int ix, int iy, float w, bool use) {
+            const int64_t idx = base + (int64_t)iy * p.sy + (int64_t)ix * p.sx;
+            if (!use) return;
+            if (OP == kProj)
+                acc = fmaf(w, __ldg(p.image_in + idx), acc);
+            else
+                atomicAdd(p.image_out + idx, OP == kBack ? w : w * L.scale);
+        });
+    }
+    if (OP == kProj) atomicAdd(p.proj_out + t, acc * L.scale);
+}
+
+// The segments seg[0, n_seg) of a slab of slices [S0, S1), one per lane.
+template <int OP, int P>
+__device__ __forceinline__ void walk_segments(const TorParams &p, const SegPlan &sp,
+                                              const SlabView &v, const int *seg, int n_seg,
+                                              int S0, int S1, int64_t img0) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr int kStep = slab_threads(OP);
+    for (int q0 = warp * 32; q0 < n_seg; q0 += kStep) {
+        SegLor L;
+        L.bxv = L.byv = 0.0f;
+        int a = 0, cnt = 0, w = 1, h = 1;
+        int t = -1;
+        const int q = q0 + lane;
+        if (q < n_seg) {
+            t = __ldg(seg + q);
+            if (q + kStep < n_seg) {  // the next round's record on its way to L2
+                const int u = __ldg(seg + q + kStep);
+                asm volatile("prefetch.global.L2 [%0];" :: "l"(sp.rec + u));
+            }
+            seg_lor(sp.rec, t, L);
+            if (seg_value<OP>(p, t, L)) {
+                if (!L.general) {
+                    a = max(L.s_lo, S0);
+                    cnt = max(0, min(L.s_hi, S1 - 1) - a + 1);
+                    a -= S0;
+                    // columns and rows of its largest box (voxel centres within b)
+                    w = 1 + (int)fminf(2.0f * L.bxv, (float)(P - 1));
+                    h = 1 + (int)fminf(2.0f * L.byv, (float)(P - 1));
+                } else {
+                    general_segment<OP, P>(p, t, S0, S1, v.R0, v.R1, img0);
+                }
+            }
+        }
+        __syncwarp();
+        const int n_max = __reduce_max_sync(0xffffffffu, cnt);
+        w = __reduce_max_sync(0xffffffffu, cnt > 0 ? w : 1);
+        h = __reduce_max_sync(0xffffffffu, cnt > 0 ? h : 1);
+        const bool clipped = __any_sync(
+            0xffffffffu, cnt > 0 && !(L.bxv < p.fit && L.byv < p.fit));
+        float acc = 0.0f;
+        if (clipped)
+            acc = walk_segment<OP, P, P, true>(p, v, L, a, cnt, n_max, P);
+        else
+            with_width<P>(w, [&](auto W) {
+                acc = walk_segment<OP, P, decltype(W)::value, false>(p, v, L, a, cnt, n_max, h);
+            });
+        if (OP == kProj && cnt > 0) atomicAdd(p.proj_out + t, acc * L.scale);
+    }
+}
+
 // Persistent pass over the slab-major segment list (all TOR ops but the count). Scatter
 // ops accumulate into the slab with shared atomics and flush once per slab; the
 // projection gathers from the slab (loaded from the image) and adds each LOR's partial
-// sum to its output.
-// kExpand: the (LOR, slice) items of a warp's 32 segments are spread over its lanes, 32
-// at a time (one item per lane, the LOR's constants read from its record); otherwise
-// each lane walks its own segment's slices.
-// kBand: the slabs are bands of rows (sp.nbands > 1), so rows are limited to the band.
-template <int OP, int P, bool kExpand, bool kBand>
-__global__ void __launch_bounds__(kSlabThreads, 1) tor_slab_kernel(const TorParams p, SegPlan sp) {
-    extern __shared__ float slab[];
-    __shared__ signed char owner_tab[kSlabThreads / 32][32];
+// sum to its output. One segment per lane.
+template <int OP, int P>
+__global__ void __launch_bounds__(slab_threads(OP), 1)
+tor_slab_kernel(const __grid_constant__ TorParams p, const __grid_constant__ SegPlan sp) {
+    extern __shared__ float smem[];
+    float *const zs = smem;  // [nsl] planes of the slab's slices
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    constexpr int kWarps = kSlabThreads / 32;
+    constexpr int kThreads = slab_threads(OP), kWarps = kThreads / 32;
     constexpr int pad = P - 1;
-    const int rs = slab_row_stride(p.gx, pad), ss = slab_slice_stride(p.gx, sp.band_rows, pad);
+    SlabView v;
+    v.mem = smem + sp.nsl;
+    v.zs = zs;
+    v.rs = slab_row_stride(p.gx, pad);
+    v.ss = slab_slice_stride(p.gx, sp.band_rows, pad);
+    const int rs = v.rs, ss = v.ss;
     const int origin = slab_origin(p.gx, pad);
+    float *const slab = v.mem;
     const int64_t total = sp.slab_offs[sp.n_slabs];
     const int64_t g = blockIdx.x, G = gridDim.x;
     const int64_t lo = total * g / G, hi = total * (g + 1) / G;
     if (lo >= hi) return;
     if (OP == kProj) {
-        // The padding columns stay zero: the slab loads below write grid voxels only.
+        // The padding stays zero: the slab loads below write grid voxels, and zeros to the
+        // rows that a short last band leaves over.
         const int n = slab_floats(sp.nsl, p.gx, sp.band_rows, pad);
-        for (int i = threadIdx.x; i < n; i += kSlabThreads) slab[i] = 0.0f;
+        for (int i = threadIdx.x; i < n; i += kThreads) slab[i] = 0.0f;
         __syncthreads();
     }
     int k = 0;
@@ -1201,130 +1448,38 @@ __global__ void __launch_bounds__(kSlabThreads, 1) tor_slab_kernel(const TorPara
         const int R0 = band * sp.band_rows, R1 = min(R0 + sp.band_rows, p.gy);
         const int nbr = R1 - R0;
         const int64_t img0 = (int64_t)fr * p.frame_stride;
-        const int n_rows = (S1 - S0) * nbr;
+        v.R0 = R0;
+        v.R1 = R1;
+        v.base = (unsigned)(origin - R0 * rs) - kMagicBits * (unsigned)(rs + 1);
+        const int *seg = sp.seg + pos;
+        const int n_seg = (int)(end - pos);  // a list holds fewer than 2^31 entries
+        for (int i = threadIdx.x; i < S1 - S0; i += kThreads) zs[i] = slice_z<OP>(p, S0 + i);
         if (OP == kProj) {
             const float *src = p.image_in + img0 + (int64_t)S0 * p.sz + (int64_t)R0 * p.sy;
-            for (int r = warp; r < n_rows; r += kWarps) {
-                const int sl = r / nbr, iy = r - sl * nbr;
+            const int rows = min(nbr + pad, sp.band_rows);  // past the grid's end: zeros
+            for (int r = warp; r < (S1 - S0) * rows; r += kWarps) {
+                const int sl = r / rows, iy = r - sl * rows;
                 const float *g = src + (int64_t)sl * p.sz + (int64_t)iy * p.sy;
                 float *d = slab + origin + sl * ss + iy * rs;
-                for (int ix = lane; ix < p.gx; ix += 32) d[ix] = __ldg(g + (int64_t)ix * p.sx);
+                for (int ix = lane; ix < p.gx; ix += 32)
+                    d[ix] = iy < nbr ? __ldg(g + (int64_t)ix * p.sx) : 0.0f;
             }
         } else {
             const int n = slab_floats(S1 - S0, p.gx, sp.band_rows, pad);
-            for (int i = threadIdx.x; i < n; i += kSlabThreads) slab[i] = 0.0f;
+            for (int i = threadIdx.x; i < n; i += kThreads) slab[i] = 0.0f;
         }
         __syncthreads();
-        for (int64_t q0 = pos + (int64_t)warp * 32; q0 < end; q0 += (int64_t)kWarps * 32) {
-            const int64_t q = q0 + lane;
-            LorConst L;
-            int a = 0, cnt = 0, t = -1;
-            if (q < end) {
-                t = sp.seg[q];
-                if (lor_load<OP>(p, sp.rec, t, L)) {
-                    a = max(L.s_lo, S0);
-                    cnt = max(0, min(L.s_hi, S1 - 1) - a + 1);
-                }
-            }
-            if (!kExpand) {
-                float acc = 0.0f;
-                for (int i = 0; i < cnt; i++) {
-                    const int s = a + i;
-                    float *sb = slab + origin + (s - S0) * ss;  // slice s, row R0
-                    if (OP == kProj) {
-                        slice_visit<OP, P, true, kBand>(p, L, s, R0, R1,
-                                                 [&](int ix, int iy, float w, bool use) {
-                            const float v = sb[(iy - R0) * rs + ix];
-                            acc = use ? fmaf(w, v, acc) : acc;
-                        });
-                    } else {
-                        slice_visit<OP, P, true, kBand>(p, L, s, R0, R1,
-                                                 [&](int ix, int iy, float w, bool use) {
-                            if (use)
-                                atomicAdd(&sb[(iy - R0) * rs + ix], OP == kBack ? w : w * L.scale);
-                        });
-                    }
-                }
-                if (OP == kProj && cnt > 0) atomicAdd(p.proj_out + t, acc * L.scale);
-                continue;
-            }
-            int incl = cnt;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int v = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += v;
-            }
-            const int excl = incl - cnt;
-            const int n_items = __shfl_sync(0xffffffffu, incl, 31);
-            for (int base = 0; base < n_items; base += 32) {
-                for (int i = max(excl, base); i < min(incl, base + 32); ++i)
-                    owner_tab[warp][i - base] = (signed char)lane;
-                __syncwarp();
-                const int item = base + lane;
-                const bool valid = item < n_items;
-                const int o = valid ? (int)owner_tab[warp][lane] : 0;
-                __syncwarp();
-                const int a_o = __shfl_sync(0xffffffffu, a, o);
-                const int excl_o = __shfl_sync(0xffffffffu, excl, o);
-                const int t_o = __shfl_sync(0xffffffffu, t, o);
-                // the item's LOR from its record (the lanes of one LOR read the same 64
-                // bytes, served once by L1), its value scale from the owning lane
-                LorConst M;
-                const float scale_o = __shfl_sync(0xffffffffu, L.scale, o);
-                const float k0s_o = __shfl_sync(0xffffffffu, L.k0s, o);
-                const bool all_o = OP == kMap && __shfl_sync(0xffffffffu, (int)L.all, o);
-                if (valid) {
-                    lor_rec_geometry(sp.rec, t_o, M);
-                    M.scale = scale_o;
-                    M.k0s = k0s_o;
-                    M.all = all_o;
-                    if (all_o) M.bxv = M.byv = 1.0e9f;
-                }
-                float partial = 0.0f;
-                if (valid) {
-                    const int s = a_o + (item - excl_o);
-                    float *sb = slab + origin + (s - S0) * ss;  // slice s, row R0
-                    if (OP == kProj) {
-                        float acc = 0.0f;
-                        slice_visit<OP, P, true, kBand>(p, M, s, R0, R1,
-                                                 [&](int ix, int iy, float w, bool use) {
-                            const float v = sb[(iy - R0) * rs + ix];
-                            acc = use ? fmaf(w, v, acc) : acc;
-                        });
-                        partial = acc * M.scale;
-                    } else {
-                        slice_visit<OP, P, true, kBand>(p, M, s, R0, R1,
-                                                 [&](int ix, int iy, float w, bool use) {
-                            if (use)
-                                atomicAdd(&sb[(iy - R0) * rs + ix], OP == kBack ? w : w * M.scale);
-                        });
-                    }
-                }
-                if (OP == kProj) {
-                    // items of one LOR sit in consecutive lanes: segmented suffix sum
-                    const int key = valid ? o : -1 - lane;
-                    float v = partial;
-#pragma unroll
-                    for (int d = 1; d < 32; d <<= 1) {
-                        const float nv = __shfl_down_sync(0xffffffffu, v, d);
-                        const int nk = __shfl_down_sync(0xffffffffu, key, d);
-                        if (lane + d < 32 && nk == key) v += nv;
-                    }
-                    const int prev = __shfl_up_sync(0xffffffffu, key, 1);
-                    if (valid && (lane == 0 || prev != key)) atomicAdd(p.proj_out + t_o, v);
-                }
-            }
-        }
+        walk_segments<OP, P>(p, sp, v, seg, n_seg, S0, S1, img0);
         __syncthreads();
         if (OP != kProj) {
             float *out = p.image_out + img0 + (int64_t)S0 * p.sz + (int64_t)R0 * p.sy;
-            for (int r = warp; r < n_rows; r += kWarps) {
+            for (int r = warp; r < (S1 - S0) * nbr; r += kWarps) {
                 const int sl = r / nbr, iy = r - sl * nbr;
                 const float *src = slab + origin + sl * ss + iy * rs;
                 float *g = out + (int64_t)sl * p.sz + (int64_t)iy * p.sy;
                 for (int ix = lane; ix < p.gx; ix += 32) {
-                    const float v = src[ix];
-                    if (v != 0.0f) atomicAdd(g + (int64_t)ix * p.sx, v);
+                    const float val = src[ix];
+                    if (val != 0.0f) atomicAdd(g + (int64_t)ix * p.sx, val);
                 }
             }
             __syncthreads();
@@ -1385,13 +1540,28 @@ int tor_setup(TorParams &p, const int *grid, const float *center, const float *s
     // ~1e-6 (patch * inter)^2 of the exact value, the margin is 2^-16 (patch * inter)^2.
     const float span = (float)p.patch * std::max(p.inter_x, p.inter_y);
     p.box_e = span * span * (1.0f / 65536.0f);
+    p.box_x0 = -p.l_bound * p.inv_x - 0.5f;
+    p.box_y0 = -p.b_bound * p.inv_y - 0.5f;
+    p.fit = std::min((float)p.half + 0.5f, (float)(p.patch - p.half) - 0.5f) - 1.0f / 1024.0f;
+    auto twice = [](float a) {
+        unsigned u;
+        std::memcpy(&u, &a, sizeof u);
+        F2 r;
+        r.v = (unsigned long long)u << 32 | u;
+        return r;
+    };
+    p.pc.ix = twice(p.inter_x);
+    p.pc.iy = twice(p.inter_y);
+    p.pc.lb = twice(p.l_bound);
+    p.pc.bb = twice(p.b_bound);
+    p.pc.one = twice(1.0f);
+    for (int c = 0; c < 8; c++) p.pc.col[c] = twice((float)c + 0.5f);
     p.n = n;
     p.stride = lor_stride;
     // Kernel family: the shared-memory slab kernels unless tuning selects the LOR-centric
     // ones (gathers from L2, global atomics; also the fallback when a slice does not fit).
     const int path = g_tune_path.load(std::memory_order_relaxed);
     p.use_slab = path == 2 ? 0 : 1;
-    p.slab_expand = path == 3 ? 1 : 0;
     return SRF_OK;
 }
 
@@ -1410,13 +1580,13 @@ constexpr int kMinSlabSlices = 4;
 constexpr int kMinBandRows = 8;
 
 bool slab_geometry(const TorParams &p, int pad, SegPlan &sp) {
-    if (p.gx > (1 << 14) || p.gy > (1 << 14)) return false;
+    if (p.gx > (1 << 14) || p.gy > (1 << 14) || p.gz > kSliceMask) return false;
     const size_t budget = kSlabSmemBytes / sizeof(float);
     auto fits = [&](int n, int rows) {
         return (size_t)slab_floats(n, p.gx, rows, pad) <= budget;
     };
     int full = 0;
-    while (full < p.gz && fits(full + 1, p.gy)) full++;
+    while (full < std::min(p.gz, kMaxSlabSlices) && fits(full + 1, p.gy)) full++;
     const int want = g_tune_nsl.load(std::memory_order_relaxed);
     if ((want == 0 && full >= std::min(kMinSlabSlices, p.gz)) || (want > 0 && want <= full)) {
         sp.nsl = want > 0 ? want : full;
@@ -1477,20 +1647,16 @@ TorParams lor_chunk(const TorParams &p, int64_t c0, int64_t n) {
     return q;
 }
 
-// The slab kernel instance for p's variant, with its shared-memory limit raised once per
-// device.
+// The slab kernel instance, with its shared-memory limit raised once per device.
 template <int OP, int P>
-int slab_kernel(const TorParams &p, bool band, void (**kern)(const TorParams, SegPlan)) {
-    *kern = p.slab_expand
-                ? (band ? tor_slab_kernel<OP, P, true, true> : tor_slab_kernel<OP, P, true, false>)
-                : (band ? tor_slab_kernel<OP, P, false, true> : tor_slab_kernel<OP, P, false, false>);
-    static std::atomic<unsigned long long> attr_set[4];  // per kernel instance, per device
-    std::atomic<unsigned long long> &done = attr_set[(p.slab_expand ? 2 : 0) + (band ? 1 : 0)];
+int slab_kernel(void (**kern)(const TorParams, const SegPlan)) {
+    *kern = tor_slab_kernel<OP, P>;
+    static std::atomic<unsigned long long> done{0};  // per device
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
     if (!(done.load() & (1ull << dev))) {
         const cudaError_t e = cudaFuncSetAttribute(
-            *kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSlabSmemBytes);
+            *kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSlabSmemMax);
         if (e != cudaSuccess) {
             set_cuda_error(e);
             return SRF_ERR_CUDA;
@@ -1543,17 +1709,18 @@ int launch_slab(const TorParams &p, const TorParams *p2, cudaStream_t stream) {
     sp.seg = reinterpret_cast<int *>(w2 + b_range + b_counts + b_offs + b_slab);
 
     const bool band = sp.nbands > 1;
-    void (*kern)(const TorParams, SegPlan) = nullptr;
-    void (*kern2)(const TorParams, SegPlan) = nullptr;
-    int st = slab_kernel<OP, P>(p, band, &kern);
+    void (*kern)(const TorParams, const SegPlan) = nullptr;
+    void (*kern2)(const TorParams, const SegPlan) = nullptr;
+    int st = slab_kernel<OP, P>(&kern);
     if constexpr (OP2 >= 0) {
-        if (st == SRF_OK) st = slab_kernel<OP2, P>(*p2, band, &kern2);
+        if (st == SRF_OK) st = slab_kernel<OP2, P>(&kern2);
     }
     if (st != SRF_OK) {
         cudaFreeAsync(ws, stream);
         return st;
     }
-    const size_t smem = sizeof(float) * (size_t)slab_floats(sp.nsl, p.gx, sp.band_rows, P - 1);
+    const size_t smem =
+        sizeof(float) * ((size_t)slab_floats(sp.nsl, p.gx, sp.band_rows, P - 1) + sp.nsl);
     int64_t *slab_tot = sp.slab_offs + sp.n_slabs + 1;
     if (OP == kProj) {
         e = cudaMemsetAsync(p.proj_out, 0, sizeof(float) * p.n, stream);
@@ -1580,10 +1747,10 @@ int launch_slab(const TorParams &p, const TorParams *p2, cudaStream_t stream) {
             seg_fill_kernel<true><<<sq.ntiles, kSegThreads, fill_bytes, stream>>>(q, sq);
         else
             seg_fill_kernel<false><<<sq.ntiles, kSegThreads, fill_bytes, stream>>>(q, sq);
-        kern<<<num_sms() * mult, kSlabThreads, smem, stream>>>(q, sq);
+        kern<<<num_sms() * mult, slab_threads(OP), smem, stream>>>(q, sq);
         count_launches(5);
         if constexpr (OP2 >= 0) {
-            kern2<<<num_sms() * mult, kSlabThreads, smem, stream>>>(
+            kern2<<<num_sms() * mult, slab_threads(OP2), smem, stream>>>(
                 lor_chunk(*p2, c0, std::min(chunk, p.n - c0)), sq);
             count_launches(1);
         }
@@ -1600,9 +1767,9 @@ int launch_slab(const TorParams &p, const TorParams *p2, cudaStream_t stream) {
 template <int OP>
 int tor_launch(TorParams &p, cudaStream_t stream, bool generic = false) {
     if (p.n == 0) return SRF_OK;
-    if ((OP == kProj || OP == kBack || OP == kMap || OP == kAdj) && !generic && p.use_slab) {
+    if constexpr (OP != kCount) {
         int st = -1;
-        switch (p.patch) {
+        switch (generic || !p.use_slab ? 0 : p.patch) {
             case 2: st = launch_slab<OP, 2, -1>(p, nullptr, stream); break;
             case 3: st = launch_slab<OP, 3, -1>(p, nullptr, stream); break;
             case 4: st = launch_slab<OP, 4, -1>(p, nullptr, stream); break;

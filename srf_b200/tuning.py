@@ -2,8 +2,7 @@
 
 ``set_tuning(path, slab_slices, grid_mult)`` sets the library's process-wide knobs
 (``srf_tor_set_tuning``): the kernel family (0 automatic, 1 shared-memory slabs with a
-lane per (LOR, slab) segment, 2 LOR-centric, 3 shared-memory slabs with a segment's
-slices spread over lanes), the number of slices per shared-memory slab (0 = as many as fit) and
+lane per (LOR, slab) segment, 2 LOR-centric, 3 the same as 1), the number of slices per shared-memory slab (0 = as many as fit) and
 the grid multiplier of the persistent slab kernel (0 = automatic). ``set_tuning()``
 restores the library's defaults (all automatic).
 
@@ -45,8 +44,8 @@ def set_scratch_limit(nbytes=0):
 def candidates(max_slab_slices):
     """Settings worth trying: full and half-depth slabs, each with the library's automatic
     grid multiplier (0: chosen per op and call size) and with multipliers 1 and 2 fixed,
-    the spread-items slab kernel and the LOR-centric kernels. The automatic choice comes
-    first, so a tie keeps it."""
+    path 3 (the slab kernels again, kept for stored settings) and the LOR-centric kernels.
+    The automatic choice comes first, so a tie keeps it."""
     out = [(1, 0, 0), (1, 0, 1), (1, 0, 2)]
     half = max(1, max_slab_slices // 2)
     if half < max_slab_slices:
