@@ -854,7 +854,7 @@ __global__ void __launch_bounds__(256) tor_kernel_p(const TorParams p) {
 //
 // Binning (three kernels, deterministic counts, order inside a slab unspecified):
 //   seg_count  per LOR: slab range -> packed (k_lo, k_hi); per-tile slab histogram
-//   seg_scan   per slab: scan over tiles; slab offsets; total
+//   seg_scan   per slab: scan over tiles; the last block: slab offsets; total
 //   seg_fill   per LOR: write its index into each slab's list
 
 constexpr int kSegThreads = 512;
@@ -879,6 +879,7 @@ std::atomic<long long> g_seg_scratch_bytes{kSegScratchDefault};
 
 struct SegPlan {
     int nsl, n_slabs, ntiles;  // n_slabs counts slab ids over all frames
+    int items;                 // a tile is items x kSegThreads LORs
     int slabs_pf;              // slice ranges per frame
     int nbands, band_rows;     // row bands per slice range and rows per band (last: fewer)
     unsigned band_magic;       // ceil(2^32 / band_rows): r / band_rows = umulhi(r, magic)
@@ -886,27 +887,34 @@ struct SegPlan {
     int *tile_counts;      // [ntiles * n_slabs]
     int64_t *tile_offs;    // [ntiles * n_slabs]
     int64_t *slab_offs;    // [n_slabs + 1]
+    int64_t *slab_tot;     // [n_slabs]
+    unsigned *scanned;     // slabs that seg_scan has finished
     int *seg;              // [capacity] LOR indices, slab-major
     LorRec *rec;           // [n] per-LOR records written by seg_count
 };
 
 // Slab ids (slice range k of a LOR's frame, row band b): id = k * nbands + b, with k
-// counted over frames. With row bands, the bands of slice range k are those the LOR's
-// window rows can reach in its slices there: the rows follow the crossing point's y, which
-// is monotonic in the slice, so the rows of the range's two end slices, with two rows of
-// margin and the window's extent, bound them. y1, z1, d1 = y2 - y1 and dz = z2 - z1 come
-// from the LOR's record, so counting and filling agree bit for bit.
+// counted over frames. With row bands, the bands of slice range k are those that hold a
+// voxel of the tube's section in the LOR's slices there: the rows follow the crossing point's
+// y, which is monotonic in the slice, so the rows of the range's two end slices, with the
+// box's half-extent (at most the window's reach) and a margin far above the rounding here,
+// bound them. (Not the window's rows with two more on either side, which put LORs into
+// bands they add nothing to: 4M events at 256 x 256 x 128 12.31 -> 11.52 ms.) y1, z1, d1 = y2 - y1,
+// dz = z2 - z1 and the half-extent come from the LOR's record, so counting and filling agree
+// bit for bit.
 struct SlabIdLor {
     int k_lo, k_hi, s_lo, s_hi, f0;
     float y1, d1, r0, rs, z1, dz;
+    float reach;  // rows above and below the crossing
     int lin;  // y at slice s from r0 + s rs (else the division, where 1 / dz would overflow)
 };
 
 __device__ __forceinline__ SlabIdLor slab_id_lor(const TorParams &p, const SegPlan &sp,
                                                  int64_t t, int k_lo, int k_hi, int s_lo,
                                                  int s_hi, float y1, float z1, float d1,
-                                                 float dz) {
+                                                 float dz, float byv) {
     SlabIdLor c;
+    c.reach = fminf(byv, (float)p.patch + 1.0f) + 0.02f;
     c.k_lo = k_lo;
     c.k_hi = k_hi;
     c.s_lo = s_lo;
@@ -943,10 +951,10 @@ __device__ __forceinline__ void range_slab_ids(const TorParams &p, const SegPlan
     const float lo = fminf(ya, yb), hi = fmaxf(ya, yb);
     int b_lo = 0, b_hi = sp.nbands - 1;
     if (lo == lo && hi == hi) {  // else: every band, left to the exact per-slice test
-        const float flo = fminf(fmaxf(floorf((lo - p.b_bound) * p.inv_y), -1.0e8f), 1.0e8f);
-        const float fhi = fminf(fmaxf(floorf((hi - p.b_bound) * p.inv_y), -1.0e8f), 1.0e8f);
-        const int r_lo = max((int)flo - p.half - 2, 0);
-        const int r_hi = min((int)fhi - p.half + p.patch + 1, p.gy - 1);
+        const float flo = ceilf(fmaf(lo - p.b_bound, p.inv_y, -0.5f) - c.reach);
+        const float fhi = floorf(fmaf(hi - p.b_bound, p.inv_y, -0.5f) + c.reach);
+        const int r_lo = (int)fmaxf(fminf(flo, 1.0e8f), 0.0f);
+        const int r_hi = (int)fminf(fmaxf(fhi, -1.0f), (float)(p.gy - 1));
         if (r_lo > r_hi) return;
         // 0 <= r < 2^14 and band_rows < 2^14: the multiply-high quotient is exact
         b_lo = (int)__umulhi((unsigned)r_lo, sp.band_magic);
@@ -996,6 +1004,7 @@ __device__ __forceinline__ void warp_slab_ids(const TorParams &p, const SegPlan 
             m.rs = __shfl_sync(0xffffffffu, c.rs, o);
             m.z1 = __shfl_sync(0xffffffffu, c.z1, o);
             m.dz = __shfl_sync(0xffffffffu, c.dz, o);
+            m.reach = __shfl_sync(0xffffffffu, c.reach, o);
         }
         if (valid) range_slab_ids<kBand>(p, sp, m, k, [&](int id) { g(id, to); });
     }
@@ -1028,9 +1037,10 @@ __global__ void __launch_bounds__(kSegThreads) seg_count_kernel(const TorParams 
     extern __shared__ int hist[];  // [n_slabs]
     __shared__ signed char owner_tab[kSegThreads / 32][32];
     for (int k = threadIdx.x; k < sp.n_slabs; k += kSegThreads) hist[k] = 0;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *sp.scanned = 0;
     __syncthreads();
-    const int64_t base = (int64_t)blockIdx.x * kSegTile;
-    for (int it = 0; it < kSegItems; it++) {
+    const int64_t base = (int64_t)blockIdx.x * (sp.items * kSegThreads);
+    for (int it = 0; it < sp.items; it++) {
         const int64_t t = base + (int64_t)it * kSegThreads + threadIdx.x;
         if (base + (int64_t)it * kSegThreads >= p.n) break;  // warp-uniform (whole block)
         int packed = -1;
@@ -1038,7 +1048,14 @@ __global__ void __launch_bounds__(kSegThreads) seg_count_kernel(const TorParams 
         bool ok = false;
         SlabIdLor c{};
         if (t < p.n) {
+            if (OP == kProj) p.proj_out[t] = 0.0f;  // the slab kernels add to it
             ok = geometry_any<OP>(p, t, L);  // generated map LORs are made here
+            if (OP == kMap && ok && p.values) {
+                // a zero or non-finite divisor lands on every voxel of the window
+                LorConst m = L;
+                lor_value_scale<OP>(p, t, m);
+                if (m.all) L.byv = m.byv;
+            }
             if (ok) {  // only LORs that enter the slab lists are ever read back
                 const LorRec r = make_rec(p, L, OP != kMap && p.tof_on);
                 float4 *q = reinterpret_cast<float4 *>(sp.rec + t);
@@ -1052,7 +1069,8 @@ __global__ void __launch_bounds__(kSegThreads) seg_count_kernel(const TorParams 
                 const int f0 = p.frame ? __ldg(p.frame + t) * sp.slabs_pf : 0;
                 const int k_lo = f0 + L.s_lo / sp.nsl, k_hi = f0 + L.s_hi / sp.nsl;
                 packed = k_lo | (k_hi << 16);
-                c = slab_id_lor(p, sp, t, k_lo, k_hi, L.s_lo, L.s_hi, L.y1, L.z1, L.d1, L.dz);
+                c = slab_id_lor(p, sp, t, k_lo, k_hi, L.s_lo, L.s_hi, L.y1, L.z1, L.d1, L.dz,
+                                L.byv);
             }
             sp.range[t] = packed;
         }
@@ -1069,17 +1087,16 @@ __global__ void __launch_bounds__(kSegThreads) seg_count_kernel(const TorParams 
         sp.tile_counts[(int64_t)blockIdx.x * sp.n_slabs + k] = hist[k];
 }
 
-// Per slab (one block each): exclusive scan of the tile counts -> tile_offs, slab total
-// -> slab_tot[k]. A second single-warp kernel turns the totals into slab offsets.
-__global__ void __launch_bounds__(1024) seg_scan_kernel(SegPlan sp, int64_t *slab_tot) {
-    __shared__ int64_t warp_sums[32];
-    const int k = blockIdx.x;
+// The calling block's exclusive scan of v(0 .. n - 1), put(i, sum before i) for each;
+// returns the total. All 1024 threads of the block call it.
+template <typename V, typename Put>
+__device__ __forceinline__ int64_t block_scan(int n, int64_t (&warp_sums)[32], V &&v, Put &&put) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     int64_t carry = 0;
-    for (int start = 0; start < sp.ntiles; start += 1024) {
-        const int tile = start + threadIdx.x;
-        const int64_t v = tile < sp.ntiles ? sp.tile_counts[(int64_t)tile * sp.n_slabs + k] : 0;
-        int64_t x = v;
+    for (int start = 0; start < n; start += 1024) {
+        const int i = start + threadIdx.x;
+        const int64_t mine = i < n ? v(i) : 0;
+        int64_t x = mine;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const int64_t y = __shfl_up_sync(0xffffffffu, x, o);
@@ -1097,24 +1114,36 @@ __global__ void __launch_bounds__(1024) seg_scan_kernel(SegPlan sp, int64_t *sla
             warp_sums[lane] = w;
         }
         __syncthreads();
-        const int64_t before = (wid ? warp_sums[wid - 1] : 0) + carry;
-        if (tile < sp.ntiles) sp.tile_offs[(int64_t)tile * sp.n_slabs + k] = before + x - v;
-        const int64_t chunk = warp_sums[31];
+        if (i < n) put(i, (wid ? warp_sums[wid - 1] : 0) + carry + x - mine);
+        carry += warp_sums[31];
         __syncthreads();
-        carry += chunk;
     }
-    if (threadIdx.x == 0) slab_tot[k] = carry;
+    return carry;
 }
 
-__global__ void seg_offsets_kernel(SegPlan sp, const int64_t *slab_tot) {
+// Per slab (one block each): exclusive scan of the tile counts -> tile_offs, slab total
+// -> slab_tot[k]. The last block to finish scans the totals into the slab offsets (a
+// kernel of its own, with one thread adding them up, took 3 to 12 us).
+__global__ void __launch_bounds__(1024) seg_scan_kernel(const SegPlan sp) {
+    __shared__ int64_t warp_sums[32];
+    __shared__ bool last;
+    const int k = blockIdx.x;
+    const int64_t total = block_scan(
+        sp.ntiles, warp_sums,
+        [&](int i) { return (int64_t)sp.tile_counts[(int64_t)i * sp.n_slabs + k]; },
+        [&](int i, int64_t before) { sp.tile_offs[(int64_t)i * sp.n_slabs + k] = before; });
     if (threadIdx.x == 0) {
-        int64_t acc = 0;
-        for (int k = 0; k < sp.n_slabs; k++) {
-            sp.slab_offs[k] = acc;
-            acc += slab_tot[k];
-        }
-        sp.slab_offs[sp.n_slabs] = acc;
+        sp.slab_tot[k] = total;
+        __threadfence();
+        last = atomicAdd(sp.scanned, 1u) == (unsigned)sp.n_slabs - 1u;
     }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    const int64_t all = block_scan(
+        sp.n_slabs, warp_sums, [&](int i) { return __ldcg(sp.slab_tot + i); },
+        [&](int i, int64_t before) { sp.slab_offs[i] = before; });
+    if (threadIdx.x == 0) sp.slab_offs[sp.n_slabs] = all;
 }
 
 // Filling: one LOR per lane, so that the lanes of a warp that meet a slab append their
@@ -1132,15 +1161,15 @@ __global__ void __launch_bounds__(kSegThreads) seg_fill_kernel(const TorParams p
         tile_base[k] = sp.slab_offs[k] + sp.tile_offs[(int64_t)blockIdx.x * sp.n_slabs + k];
     }
     __syncthreads();
-    const int64_t base = (int64_t)blockIdx.x * kSegTile;
-    for (int it = 0; it < kSegItems; it++) {
+    const int64_t base = (int64_t)blockIdx.x * (sp.items * kSegThreads);
+    for (int it = 0; it < sp.items; it++) {
         const int64_t t = base + (int64_t)it * kSegThreads + threadIdx.x;
         if (t >= p.n) break;
         const int packed = sp.range[t];
         if (packed < 0) continue;
         const int k_lo = packed & 0xffff, k_hi = packed >> 16;
         int s_lo = 0, s_hi = p.gz - 1;
-        float y1 = 0.f, z1 = 0.f, d1 = 0.f, dz = 1.f;
+        float y1 = 0.f, z1 = 0.f, d1 = 0.f, dz = 1.f, byv = 0.f;
         if (kBand) {  // the values seg_count used, from the LOR's record
             const float4 *q = reinterpret_cast<const float4 *>(sp.rec + t);
             const float4 a = q[0], b = q[1], d = q[3];
@@ -1151,8 +1180,10 @@ __global__ void __launch_bounds__(kSegThreads) seg_fill_kernel(const TorParams p
             z1 = a.z;
             d1 = b.x;
             dz = b.y;
+            byv = q[2].w;
         }
-        const SlabIdLor c = slab_id_lor(p, sp, t, k_lo, k_hi, s_lo, s_hi, y1, z1, d1, dz);
+        const SlabIdLor c =
+            slab_id_lor(p, sp, t, k_lo, k_hi, s_lo, s_hi, y1, z1, d1, dz, byv);
         for (int k = k_lo; k <= k_hi; k++)
             range_slab_ids<kBand>(p, sp, c, k, [&](int id) {
                 const int pos = warp_increment(cursor, id);
@@ -1871,21 +1902,27 @@ int launch_slab(const TorParams &p, const TorParams *p2, cudaStream_t stream) {
     if (!slab_geometry(p, P - 1, sp)) return -1;
     // The segment list is sized for the worst case (every LOR in every slab of its frame);
     // with each LOR's record and slab range, LORs are taken in chunks small enough that
-    // this stays within the scratch budget (at least one 4096-LOR tile per chunk).
+    // this stays within the scratch budget (at least 4096 LORs per chunk).
     const int64_t max_slabs_per_lor = (int64_t)sp.slabs_pf * sp.nbands;
     const size_t budget = (size_t)g_seg_scratch_bytes.load(std::memory_order_relaxed);
     int64_t chunk = (int64_t)(budget / (sizeof(int) * (size_t)max_slabs_per_lor +
                                         sizeof(LorRec) + sizeof(int)));
     chunk = std::max<int64_t>(kSegTile, chunk / kSegTile * kSegTile);
     chunk = std::min<int64_t>(chunk, p.n);
-    sp.ntiles = (int)((chunk + kSegTile - 1) / kSegTile);
+    // Tiles of 512 to 4096 LORs, about two per SM where the call has so many: a block works
+    // through its tile 512 LORs at a time, so a short call wants many short tiles (50k LORs
+    // on 128 x 64 slices: count and fill 21 + 18 -> 4.8 + 4.2 us) and a long one few.
+    sp.items = (int)std::min<int64_t>(
+        kSegItems, std::max<int64_t>(1, chunk / ((int64_t)kSegThreads * 2 * num_sms())));
+    const int tile = sp.items * kSegThreads;
+    sp.ntiles = (int)((chunk + tile - 1) / tile);
     // Scratch from the library's stream-ordered pool: no host synchronisation, capturable.
     const size_t cap = (size_t)chunk * (size_t)max_slabs_per_lor;
     auto al = [](size_t v) { return (v + 255) & ~(size_t)255; };
     const size_t b_range = al(sizeof(int) * chunk);
     const size_t b_counts = al(sizeof(int) * (size_t)sp.ntiles * sp.n_slabs);
     const size_t b_offs = al(sizeof(int64_t) * (size_t)sp.ntiles * sp.n_slabs);
-    const size_t b_slab = al(sizeof(int64_t) * (2 * sp.n_slabs + 1));
+    const size_t b_slab = al(sizeof(int64_t) * (2 * sp.n_slabs + 2));
     const size_t b_seg = al(sizeof(int) * cap);
     const size_t b_rec = al(sizeof(LorRec) * chunk);
     char *ws = nullptr;
@@ -1916,34 +1953,26 @@ int launch_slab(const TorParams &p, const TorParams *p2, cudaStream_t stream) {
     }
     const size_t smem =
         sizeof(float) * ((size_t)slab_floats(sp.nsl, p.gx, sp.band_rows, P - 1) + sp.nsl);
-    int64_t *slab_tot = sp.slab_offs + sp.n_slabs + 1;
-    if (OP == kProj) {
-        e = cudaMemsetAsync(p.proj_out, 0, sizeof(float) * p.n, stream);
-        if (e != cudaSuccess) {
-            set_cuda_error(e);
-            cudaFreeAsync(ws, stream);
-            return SRF_ERR_CUDA;
-        }
-    }
+    sp.slab_tot = sp.slab_offs + sp.n_slabs + 1;
+    sp.scanned = reinterpret_cast<unsigned *>(sp.slab_tot + sp.n_slabs);
     const int mult = slab_grid_mult(OP, sp, chunk);
     const size_t hist_bytes = sizeof(int) * (size_t)sp.n_slabs;  // <= 16 KB (kMaxSlabs)
     const size_t fill_bytes = (sizeof(int64_t) + sizeof(int)) * (size_t)sp.n_slabs;  // <= 48 KB
     for (int64_t c0 = 0; c0 < p.n && st == SRF_OK; c0 += chunk) {
         const TorParams q = lor_chunk(p, c0, std::min(chunk, p.n - c0));
         SegPlan sq = sp;
-        sq.ntiles = (int)((q.n + kSegTile - 1) / kSegTile);
+        sq.ntiles = (int)((q.n + tile - 1) / tile);
         if (band)
             seg_count_kernel<OP, true><<<sq.ntiles, kSegThreads, hist_bytes, stream>>>(q, sq);
         else
             seg_count_kernel<OP, false><<<sq.ntiles, kSegThreads, hist_bytes, stream>>>(q, sq);
-        seg_scan_kernel<<<sq.n_slabs, 1024, 0, stream>>>(sq, slab_tot);
-        seg_offsets_kernel<<<1, 32, 0, stream>>>(sq, slab_tot);
+        seg_scan_kernel<<<sq.n_slabs, 1024, 0, stream>>>(sq);
         if (band)
             seg_fill_kernel<true><<<sq.ntiles, kSegThreads, fill_bytes, stream>>>(q, sq);
         else
             seg_fill_kernel<false><<<sq.ntiles, kSegThreads, fill_bytes, stream>>>(q, sq);
         kern<<<num_sms() * mult, slab_threads(OP), smem, stream>>>(q, sq);
-        count_launches(5);
+        count_launches(4);
         if constexpr (OP2 >= 0) {
             kern2<<<num_sms() * mult, slab_threads(OP2), smem, stream>>>(
                 lor_chunk(*p2, c0, std::min(chunk, p.n - c0)), sq);
