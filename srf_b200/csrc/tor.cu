@@ -115,7 +115,7 @@ struct TorParams {
     float *image_out;
     float *proj_out;
     int *count_out;   // kCount: [n] voxels with non-zero weight, [n] window voxels visited
-    int use_slab;     // scatter ops: shared-memory slab kernel (1) or global atomics (0)
+    int use_slab;     // slab kernels: never (0), where they apply (1), by few_lors (2)
     float left;       // scatter ops: the weight a LOR leaves in a slice, about
     float box_x0, box_y0;  // -bound / inter - 1/2: voxel-centre units of a coordinate 0
     PairConsts pc;    // the geometry as operands of the paired arithmetic (slab kernels)
@@ -1221,6 +1221,9 @@ __device__ __forceinline__ float div_by(float a, float b, float inv_b) {
     return __fmaf_rn(__fmaf_rn(-q, b, a), inv_b, q);
 }
 
+// Words of the table of slice planes in front of the slab (the slab stays 16-byte aligned).
+__host__ __device__ __forceinline__ int slab_table(int nsl) { return (nsl + 3) & ~3; }
+
 // Where a slab sits and how its shared memory is laid out.
 struct SlabView {
     float *mem;       // the slab's words
@@ -1574,6 +1577,13 @@ __device__ __forceinline__ void walk_segments(const TorParams &p, const SegPlan 
     }
 }
 
+// Sets words [0, n) of the slab (and up to three more) to zero.
+template <int kThreads>
+__device__ __forceinline__ void clear_slab(float *slab, int n) {
+    for (int i = threadIdx.x; i < (n + 3) / 4; i += kThreads)
+        reinterpret_cast<float4 *>(slab)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+}
+
 // Persistent pass over the slab-major segment list (all TOR ops but the count). Scatter
 // ops accumulate into the slab with shared atomics and flush once per slab pass; the
 // projection gathers from the slab (loaded from the image) and adds each LOR's partial
@@ -1587,10 +1597,10 @@ tor_slab_kernel(const __grid_constant__ TorParams p, const __grid_constant__ Seg
     __shared__ Pass pass;
     float *const zs = smem;  // [nsl] planes of the slab's slices
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    constexpr int kThreads = slab_threads(OP), kWarps = kThreads / 32;
+    constexpr int kThreads = slab_threads(OP);
     constexpr int pad = P - 1;
     SlabView v;
-    v.mem = smem + sp.nsl;
+    v.mem = smem + slab_table(sp.nsl);
     v.zs = zs;
     v.rs = slab_row_stride(p.gx, pad);
     v.ss = slab_slice_stride(p.gx, sp.band_rows, pad);
@@ -1604,8 +1614,7 @@ tor_slab_kernel(const __grid_constant__ TorParams p, const __grid_constant__ Seg
     if (OP == kProj) {
         // The padding stays zero: the slab loads below write grid voxels, and zeros to the
         // rows that a short last band leaves over.
-        const int n = slab_floats(sp.nsl, p.gx, sp.band_rows, pad);
-        for (int i = threadIdx.x; i < n; i += kThreads) slab[i] = 0.0f;
+        clear_slab<kThreads>(slab, slab_floats(sp.nsl, p.gx, sp.band_rows, pad));
         __syncthreads();
     }
     int k = 0;
@@ -1638,7 +1647,7 @@ tor_slab_kernel(const __grid_constant__ TorParams p, const __grid_constant__ Seg
         if (OP == kProj) {
             const float *src = p.image_in + img0 + (int64_t)S0 * p.sz + (int64_t)R0 * p.sy;
             const int rows = min(nbr + pad, sp.band_rows);  // past the grid's end: zeros
-            for (int r = warp; r < (S1 - S0) * rows; r += kWarps) {
+            for (int r = warp; r < (S1 - S0) * rows; r += kThreads / 32) {
                 const int sl = r / rows, iy = r - sl * rows;
                 const float *g = src + (int64_t)sl * p.sz + (int64_t)iy * p.sy;
                 float *d = slab + origin + sl * ss + iy * rs;
@@ -1661,7 +1670,7 @@ tor_slab_kernel(const __grid_constant__ TorParams p, const __grid_constant__ Seg
             bool floats = !plan.fixed;
             while (at < n_seg) {
                 const int m = floats ? n_seg - at : min(len, n_seg - at);
-                for (int i = threadIdx.x; i < n; i += kThreads) slab[i] = 0.0f;
+                clear_slab<kThreads>(slab, n);
                 if (threadIdx.x < 2) sums[threadIdx.x] = 0;
                 if (threadIdx.x == 0)
                     pass = Pass{seg + at, m, S0, S1, tried - at, floats, plan, img0};
@@ -1672,8 +1681,11 @@ tor_slab_kernel(const __grid_constant__ TorParams p, const __grid_constant__ Seg
                 __syncthreads();
                 if (!floats) {  // the units added against the words' sum
                     unsigned long long words = 0;
-                    for (int i = threadIdx.x; i < n; i += kThreads)
-                        words += __float_as_uint(slab[i]);
+                    for (int i = threadIdx.x; i < (n + 3) / 4; i += kThreads) {
+                        const uint4 q = reinterpret_cast<const uint4 *>(slab)[i];
+                        words += (unsigned long long)q.x + q.y;
+                        words += (unsigned long long)q.z + q.w;
+                    }
 #pragma unroll
                     for (int o = 16; o > 0; o >>= 1) {
                         units += __shfl_xor_sync(0xffffffffu, units, o);
@@ -1695,13 +1707,19 @@ tor_slab_kernel(const __grid_constant__ TorParams p, const __grid_constant__ Seg
                 const float size = exp2f((float)(plan.exponent - plan.bits));
                 const float unit = plan.negative ? -size : size;
                 float *out = p.image_out + img0 + (int64_t)S0 * p.sz + (int64_t)R0 * p.sy;
-                for (int r = warp; r < (S1 - S0) * nbr; r += kWarps) {
+                for (int r = warp; r < (S1 - S0) * nbr; r += kThreads / 32) {
                     const int sl = r / nbr, iy = r - sl * nbr;
                     const float *src = slab + origin + sl * ss + iy * rs;
                     float *g = out + (int64_t)sl * p.sz + (int64_t)iy * p.sy;
-                    for (int ix = lane; ix < p.gx; ix += 32) {
-                        const float val = floats ? src[ix] : unit * (float)__float_as_uint(src[ix]);
-                        if (val != 0.0f) atomicAdd(g + (int64_t)ix * p.sx, val);
+                    for (int ix = lane; ix < p.gx; ix += 128) {
+#pragma unroll
+                        for (int u = 0; u < 4; u++) {
+                            const int c = ix + 32 * u;
+                            const float word = c < p.gx ? src[c] : 0.0f;
+                            const float val =
+                                floats ? word : unit * (float)__float_as_uint(word);
+                            if (val != 0.0f) atomicAdd(g + (int64_t)c * p.sx, val);
+                        }
                     }
                 }
                 at += m;
@@ -1784,10 +1802,10 @@ int tor_setup(TorParams &p, const int *grid, const float *center, const float *s
     for (int c = 0; c < 8; c++) p.pc.col[c] = twice((float)c + 0.5f);
     p.n = n;
     p.stride = lor_stride;
-    // Kernel family: the shared-memory slab kernels unless tuning selects the LOR-centric
-    // ones (gathers from L2, global atomics; also the fallback when a slice does not fit).
+    // Kernel family: the shared-memory slab kernels, or the LOR-centric ones (gathers from
+    // L2, global atomics) for few LORs, by tuning, and where a slice does not fit.
     const int path = g_tune_path.load(std::memory_order_relaxed);
-    p.use_slab = path == 2 ? 0 : 1;
+    p.use_slab = path == 2 ? 0 : (path == 0 ? 2 : 1);
     return SRF_OK;
 }
 
@@ -1859,6 +1877,21 @@ int slab_grid_mult(int op, const SegPlan &sp, int64_t lors_per_launch) {
             lors_per_launch >= kGridMult2MinLors) ? 2 : 1;
 }
 
+// Whether the LOR-centric kernels do a call sooner. A slab call costs ~45 us (projection) or
+// ~75 us (scatter) before its first LOR: four or five launches, slabs of 220 KB loaded or
+// cleared and flushed, and a lane walking up to a slab's depth of slices alone. The
+// LOR-centric kernels are one launch and take ~1e-6 us (projection) or 1.7e-6 us (scatter)
+// per LOR, window voxel and slice, so they win up to ~5e7 of those (with every slice of the
+// grid counted: LORs are not longer), four times that where the slabs outnumber the SMs and
+// a CTA goes through several. Measured, slab against LOR-centric, us per projection and
+// back-projection call: 5k LORs at 128 x 128 x 64, patch 6: 111 / 42, 10k 118 / 63 (uncut
+// LORs 141 / 117), 20k 139 / 114 (uncut 175 / 210); 40k at 64 x 64 x 32, patch 4: 143 / 62;
+// 40k at 101 x 93 x 47, patch 3: 157 / 107; 10k at 256 x 256 x 128, patch 7: 962 / 89.
+bool few_lors(const TorParams &p, const SegPlan &sp) {
+    const double work = (double)p.n * p.patch * p.patch * p.gz;
+    return work <= (sp.n_slabs > num_sms() ? 2.0e8 : 5.0e7);
+}
+
 // Events [c0, c0 + n) of p as a call of their own (same images and outputs' layout).
 TorParams lor_chunk(const TorParams &p, int64_t c0, int64_t n) {
     TorParams q = p;
@@ -1900,6 +1933,7 @@ template <int OP, int P, int OP2>
 int launch_slab(const TorParams &p, const TorParams *p2, cudaStream_t stream) {
     SegPlan sp{};
     if (!slab_geometry(p, P - 1, sp)) return -1;
+    if (p.use_slab == 2 && few_lors(p, sp)) return -1;
     // The segment list is sized for the worst case (every LOR in every slab of its frame);
     // with each LOR's record and slab range, LORs are taken in chunks small enough that
     // this stays within the scratch budget (at least 4096 LORs per chunk).
@@ -1952,7 +1986,8 @@ int launch_slab(const TorParams &p, const TorParams *p2, cudaStream_t stream) {
         return st;
     }
     const size_t smem =
-        sizeof(float) * ((size_t)slab_floats(sp.nsl, p.gx, sp.band_rows, P - 1) + sp.nsl);
+        sizeof(float) * ((((size_t)slab_floats(sp.nsl, p.gx, sp.band_rows, P - 1) + 3) & ~(size_t)3) +
+                         slab_table(sp.nsl));
     sp.slab_tot = sp.slab_offs + sp.n_slabs + 1;
     sp.scanned = reinterpret_cast<unsigned *>(sp.slab_tot + sp.n_slabs);
     const int mult = slab_grid_mult(OP, sp, chunk);

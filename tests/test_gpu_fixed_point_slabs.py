@@ -9,10 +9,20 @@ import pytest
 import torch
 
 from oracle import pyoracle as O
-from srf_b200 import ops
+from srf_b200 import ops, tuning
 from tests import _cases as K
 
 pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(autouse=True)
+def slabs():
+    """The slab kernels, whatever the number of LORs."""
+    tuning.set_tuning(1, 0, 0)
+    yield
+    tuning.set_tuning()
+
+
 TOL = 1e-5
 GRID, VOXEL, KW = [48, 44, 26], 3.2, 10.19
 SIZE = [g * VOXEL for g in GRID]
