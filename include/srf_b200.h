@@ -345,6 +345,13 @@ int srf_map_process(const float *lors, int64_t num_lors, int64_t lor_stride, flo
 
 /* ------------------------------------------------------------------------- image algebra */
 
+/* No counterpart in the reference: out[f][i][j][k] = sum over n_sources (1..3) of
+ * sources[s][f * dims[0] dims[1] dims[2] + i strides[3 s] + j strides[3 s + 1] + k strides[3 s + 2]],
+ * added in the order of the sources. Each source is n_frames dense images in some axis order
+ * (strides of a permuted contiguous image); out is contiguous and none of the sources. */
+int srf_permute_sum(float *out, const int *dims, int64_t n_frames, int n_sources,
+                    const float *const *sources, const int64_t *strides, void *stream);
+
 /* MLEM/OSEM update of model/recon_step.py:48-49: image[v] *= effinv[v] * bp[v]. */
 int srf_mlem_update(float *image, const float *effinv, const float *bp, int64_t num_voxels,
                     void *stream);

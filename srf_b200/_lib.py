@@ -60,6 +60,7 @@ SIGNATURES = {
                                    _int, _p, _p, _p, _f, _p, _int, _p], _int),
     "srf_tor_count_samples": ([_p] * 7 + [_int, _p, _p, _p, _f, _p, _i64, _i64, _p], _int),
     "srf_siddon_count_samples": ([_p] * 6 + [_p, _p, _p, _p, _i64, _i64, _p], _int),
+    "srf_permute_sum": ([_p, _p, _i64, _int, _p, _p, _p], _int),
     "srf_mlem_update": ([_p, _p, _p, _i64, _p], _int),
     "srf_preprocess_workspace_size": ([_i64], _i64),
     "srf_recon_process": ([_p, _i64, _i64, C.c_double, _p, _p, _p, _i64, _p], _int),

@@ -344,6 +344,42 @@ def mlem_update_(image, effinv, bp):
     return image
 
 
+def permutable(t):
+    """Whether ``permuted_sum`` takes ``t``: float32 on a CUDA device, three axes (or frames
+    and three axes) of a dense stack in any axis order within its frames, no gradient."""
+    if not (t.is_cuda and t.dtype == torch.float32 and t.dim() in (3, 4) and t.numel() > 0) \
+            or (t.requires_grad and torch.is_grad_enabled()):
+        return False
+    dense = 1
+    for st, n in sorted(zip(t.stride()[-3:], t.shape[-3:]), key=lambda a: (a[0], a[1])):
+        if n > 1 and st != dense:
+            return False
+        dense *= n
+    return t.dim() == 3 or t.shape[0] == 1 or t.stride(0) == dense
+
+
+def permuted_sum(views):
+    """The sum of up to three views of the same shape ([d0, d1, d2] or [F, d0, d1, d2], each
+    ``permutable``) as a contiguous tensor, in the views' order: one pass over each."""
+    import ctypes as C
+    dev = _check_cuda(*views)
+    shape = views[0].shape
+    for v in views:
+        if v.shape != shape or not permutable(v):
+            raise ValueError("permuted_sum needs dense float32 views of one shape")
+    d = [int(n) for n in shape[-3:]]
+    out = torch.empty(tuple(shape), dtype=torch.float32, device=dev)
+    strides = []
+    for v in views:  # the stride of an axis of extent 1 is free: that of a dense stack
+        strides += [int(st) if n > 1 else 1 for st, n in zip(v.stride()[-3:], d)]
+    with torch.cuda.device(dev):
+        _call(dev, "srf_permute_sum", out.data_ptr(), (C.c_int * 3)(*d),
+              int(shape[0]) if len(shape) == 4 else 1, len(views),
+              (C.c_void_p * len(views))(*[v.data_ptr() for v in views]),
+              (C.c_int64 * len(strides))(*strides), _stream(dev))
+    return out
+
+
 # ------------------------------------------------------------------ batched frames
 
 
