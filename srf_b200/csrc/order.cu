@@ -13,8 +13,6 @@
 // similar slice counts. Records with NaN sort last. The sort is a stable block radix sort,
 // so the order is deterministic.
 
-#include <atomic>
-
 #include <cub/block/block_radix_sort.cuh>
 
 #include "srf_common.cuh"
@@ -25,6 +23,9 @@ namespace {
 constexpr int kOrderThreads = 512;
 constexpr int kOrderItems = 8;
 constexpr int kOrderBlock = kOrderThreads * kOrderItems;  // 4096 records
+constexpr int kIndexBits = 12;                            // of a record's place in its block
+static_assert(kOrderBlock == 1 << kIndexBits, "");
+constexpr int kKeyBits = 17;
 
 __device__ __forceinline__ int direction_class(const float *r) {
     const float dx = r[3] - r[0], dy = r[4] - r[1], dz = r[5] - r[2];
@@ -41,84 +42,49 @@ __device__ __forceinline__ int direction_class(const float *r) {
     return ((kx * 16 + ky) << 8) | kz;
 }
 
-// Records of up to kStageCols columns: the block's records pass through shared memory, so
-// both the loads and the stores are contiguous runs (records are 28-40 bytes, so one
-// thread per record would touch a new sector per lane and column). Same keys, same
-// stable sort, same output as order_kernel.
-constexpr int kStageCols = 10;
-constexpr size_t kStageBytes = sizeof(float) * kOrderBlock * kStageCols;  // 160 KB
-
-__global__ void __launch_bounds__(kOrderThreads)
-order_staged_kernel(const float *__restrict__ in, float *__restrict__ out, int64_t n, int ncols,
-                    int64_t stride) {
-    using Sort = cub::BlockRadixSort<int, kOrderThreads, kOrderItems, int>;
-    __shared__ typename Sort::TempStorage tmp;
-    __shared__ int key_perm[kOrderBlock];  // keys by record, then source record by position
-    extern __shared__ float stage[];       // [kOrderBlock][ncols]
-    const int64_t base = (int64_t)blockIdx.x * kOrderBlock;
-    const int cnt = (int)min((int64_t)kOrderBlock, n - base);
-    const int total = cnt * ncols;
-    if (stride == ncols) {
-        const float *src = in + base * stride;
-        for (int e = threadIdx.x; e < total; e += kOrderThreads) stage[e] = src[e];
-    } else {
-        for (int e = threadIdx.x; e < total; e += kOrderThreads) {
-            const int r = e / ncols;
-            stage[e] = in[(base + r) * stride + (e - r * ncols)];
-        }
-    }
-    __syncthreads();
-    for (int j = threadIdx.x; j < kOrderBlock; j += kOrderThreads)
-        key_perm[j] = j < cnt ? direction_class(stage + j * ncols) : (256 << 8);
-    __syncthreads();
-    int key[kOrderItems], idx[kOrderItems];
-#pragma unroll
-    for (int k = 0; k < kOrderItems; k++) {
-        const int j = threadIdx.x * kOrderItems + k;  // blocked arrangement: stable order
-        key[k] = key_perm[j];
-        idx[k] = j;
-    }
-    Sort(tmp).Sort(key, idx, 0, 17);  // synchronises: every key is read before the writes below
-#pragma unroll
-    for (int k = 0; k < kOrderItems; k++) key_perm[threadIdx.x * kOrderItems + k] = idx[k];
-    __syncthreads();
-    if (stride == ncols) {
-        float *dst = out + base * stride;
-        for (int e = threadIdx.x; e < total; e += kOrderThreads) {
-            const int r = e / ncols;
-            dst[e] = stage[key_perm[r] * ncols + (e - r * ncols)];
-        }
-    } else {
-        for (int e = threadIdx.x; e < total; e += kOrderThreads) {
-            const int r = e / ncols, c = e - r * ncols;
-            out[(base + r) * stride + c] = stage[key_perm[r] * ncols + c];
-        }
-    }
-}
-
-__global__ void __launch_bounds__(kOrderThreads)
+// One block per 4096 records: the keys, a stable sort of key << 12 | place (so that the place
+// needs no array of its own), then every element of the output in order from the record it
+// comes from. The records are read twice, the second time from L2, which leaves 27 KB of
+// shared memory per block and three blocks on an SM. Passing records of up to 10 columns
+// through shared memory (160 KB) left one block per SM with too few loads in flight, and
+// wider ones a thread per record: 6M records of 7 columns 217 -> 202 us, 50k of 11 columns
+// (13 blocks: a block's own latency) 53 -> 25 us. Blocks of 1024 threads took 261 and 28 us,
+// of 256 threads 235 and 34 us.
+__global__ void __launch_bounds__(kOrderThreads, 3)
 order_kernel(const float *__restrict__ in, float *__restrict__ out, int64_t n, int ncols,
              int64_t stride) {
-    using Sort = cub::BlockRadixSort<int, kOrderThreads, kOrderItems, int>;
+    using Sort = cub::BlockRadixSort<unsigned, kOrderThreads, kOrderItems>;
     __shared__ typename Sort::TempStorage tmp;
+    __shared__ unsigned short perm[kOrderBlock];
     const int64_t base = (int64_t)blockIdx.x * kOrderBlock;
-    int key[kOrderItems], idx[kOrderItems];
+    const int cnt = (int)min((int64_t)kOrderBlock, n - base);
+    const float *src = in + base * stride;
+    unsigned key[kOrderItems];
 #pragma unroll
-    for (int k = 0; k < kOrderItems; k++) {
-        const int j = threadIdx.x * kOrderItems + k;  // blocked arrangement: stable order
-        const int64_t t = base + j;
-        idx[k] = j;
-        key[k] = t < n ? direction_class(in + t * stride) : (256 << 8);  // padding sorts last
+    for (int k = 0; k < kOrderItems; k++) {  // any arrangement: the places break ties
+        const int j = k * kOrderThreads + threadIdx.x;
+        const int c = j < cnt ? direction_class(src + j * stride) : (256 << 8);  // padding last
+        key[k] = (unsigned)c << kIndexBits | (unsigned)j;
     }
-    Sort(tmp).Sort(key, idx, 0, 17);
+    Sort(tmp).Sort(key, 0, kIndexBits + kKeyBits);
 #pragma unroll
-    for (int k = 0; k < kOrderItems; k++) {
-        const int j = threadIdx.x * kOrderItems + k;
-        const int64_t dst = base + j;
-        if (dst >= n) continue;
-        const float *src = in + (base + idx[k]) * stride;
-        float *d = out + dst * stride;
-        for (int c = 0; c < ncols; c++) d[c] = src[c];
+    for (int k = 0; k < kOrderItems; k++)
+        perm[threadIdx.x * kOrderItems + k] =
+            (unsigned short)(key[k] & (unsigned)(kOrderBlock - 1));
+    __syncthreads();
+    float *dst = out + base * stride;
+    const int64_t total = (int64_t)cnt * ncols;
+    const int dr = kOrderThreads / ncols, dc = kOrderThreads - dr * ncols;
+    int r = (int)threadIdx.x / ncols, c = (int)threadIdx.x - r * ncols;
+#pragma unroll 4
+    for (int64_t e = threadIdx.x; e < total; e += kOrderThreads) {
+        dst[r * stride + c] = __ldg(src + perm[r] * stride + c);
+        r += dr;
+        c += dc;
+        if (c >= ncols) {
+            c -= ncols;
+            r++;
+        }
     }
 }
 
@@ -134,28 +100,8 @@ extern "C" int srf_order_by_direction(const float *records, int64_t num_records,
     if (!records || !out || records == out) return SRF_ERR_INVALID_ARGUMENT;
     const int64_t blocks = (num_records + kOrderBlock - 1) / kOrderBlock;
     if (blocks > INT32_MAX) return SRF_ERR_UNSUPPORTED;
-    if (ncols <= kStageCols) {
-        static std::atomic<unsigned long long> attr_set{0};  // per device
-        int dev = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
-        if (!(attr_set.load() & (1ull << dev))) {
-            const cudaError_t e = cudaFuncSetAttribute(
-                order_staged_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                (int)kStageBytes);
-            if (e != cudaSuccess) {
-                set_cuda_error(e);
-                return SRF_ERR_CUDA;
-            }
-            attr_set.fetch_or(1ull << dev);
-        }
-        order_staged_kernel<<<(int)blocks, kOrderThreads,
-                              sizeof(float) * kOrderBlock * (size_t)ncols,
-                              (cudaStream_t)stream>>>(records, out, num_records, ncols,
-                                                      record_stride);
-    } else {
-        order_kernel<<<(int)blocks, kOrderThreads, 0, (cudaStream_t)stream>>>(
-            records, out, num_records, ncols, record_stride);
-    }
+    order_kernel<<<(int)blocks, kOrderThreads, 0, (cudaStream_t)stream>>>(
+        records, out, num_records, ncols, record_stride);
     count_launches(1);
     return check_launch();
 }
