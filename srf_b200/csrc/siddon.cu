@@ -14,6 +14,7 @@
 // voxel uses float arithmetic for the Gaussian itself. The scatter ops reduce into four
 // consecutive voxels at a time where a ray's run allows (siddon_kernel).
 
+#include <algorithm>
 #include <atomic>
 #include <cfloat>
 #include <cmath>
@@ -333,8 +334,12 @@ int siddon_setup(SiddonParams &p, const int *grid, const float *center, const fl
 template <int OP>
 int siddon_launch(const SiddonParams &p, cudaStream_t stream) {
     if (p.n == 0) return SRF_OK;
+    // A thread per ray rather than a grid that fills the chip and strides: the last of 3.3
+    // strides over 1M rays ran on a third of the threads, where blocks that finish early
+    // now make room for the next (projection 0.233 -> 0.203 ms, back-projection 0.303 ->
+    // 0.289 ms; blocks of 128 0.202 / 0.295).
     const int block = 256;
-    const int grid = stride_grid(p.n, block, 8);
+    const int grid = (int)std::min<int64_t>((p.n + block - 1) / block, 1 << 30);
     constexpr bool kScatter = OP == kBack || OP == kMap || OP == kAdj;
     const bool quad = kScatter && g_sid_path.load(std::memory_order_relaxed) == 0 &&
                       (reinterpret_cast<uintptr_t>(p.image_out) & 15u) == 0 &&
