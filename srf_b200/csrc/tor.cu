@@ -10,10 +10,11 @@
 //       / sqrt(2 pi tof_sigma2)                                               (:84-91)
 // with C the LOR's TOF centre.
 //
-// Kernel structure (one launch per call instead of the reference's one launch per
-// slice): one warp per LOR, lanes over the LOR's crossed slices. Each lane computes
-// its slice's crossing point and window exactly as the reference does (the discrete
-// choices), then walks the window. The two Gaussians are folded into one exponent
+// Two kernel families instead of the reference's one launch per slice: LOR-centric (one
+// warp per LOR, lanes over its crossed slices, the image in global memory; few LORs) and
+// slabs (a lane per LOR and stretch of slices, the image in shared memory; the rest). Each
+// lane makes its slice's discrete choices (crossing, window, cut-off) exactly as the
+// reference does, then walks the tube's box in the window. The two Gaussians are folded into one exponent
 //   log2 w = d^2 * k1 + k0(slice),  k1 = log2(e)/2 (1/tse - 1/tsc),
 //   k0 = -log2(e)/2 |C - X|^2 / tse,
 // so each non-zero voxel costs one exp2; the constant tof_bin/sqrt(2 pi tof_sigma2)
@@ -861,9 +862,11 @@ constexpr int kSegThreads = 512;
 constexpr int kSegItems = 8;
 constexpr int kSegTile = kSegThreads * kSegItems;
 constexpr int kMaxSlabs = 4096;
+// Threads of a slab CTA (one CTA per SM): 72 registers each, the fewest that spill little in
+// the voxel loops. 640 / 768 / 896 / 1024 threads took 5.17 / 5.06 / 5.07 / 5.80 ms (projection)
+// and 7.09 / 6.94 / 6.77 / 7.27 ms (back-projection) for 10M events at 128 x 128 x 64.
 constexpr int kProjThreads = 896;
 constexpr int kScatThreads = 896;
-// Threads of a slab CTA (one CTA per SM).
 constexpr int slab_threads(int op) { return op == kProj ? kProjThreads : kScatThreads; }
 constexpr size_t kSlabSmemBytes = 220 * 1024;  // of the 227 KB a CTA can opt into
 constexpr int kMaxSlabSlices = 1024;           // entries of the slab's table of slice planes
@@ -965,48 +968,6 @@ __device__ __forceinline__ void range_slab_ids(const TorParams &p, const SegPlan
     for (int b = b_lo; b <= b_hi; b++) g(k * sp.nbands + b);
 }
 
-// The slab ids of the warp's LORs (lane l holds LOR t_l, `ok` when it enters the lists),
-// as (LOR, slice range) items spread over the lanes 32 at a time: g(id, t) for each. A LOR
-// meets tens of slice ranges, in numbers that differ from lane to lane, so one LOR per
-// lane would leave most lanes idle. Called by all 32 lanes of the warp.
-template <bool kBand, typename G>
-__device__ __forceinline__ void warp_slab_ids(const TorParams &p, const SegPlan &sp,
-                                              signed char (&owner)[32], bool ok, int t,
-                                              const SlabIdLor &c, G &&g) {
-    const int lane = threadIdx.x & 31;
-    const int cnt = ok ? c.k_hi - c.k_lo + 1 : 0;
-    int incl = cnt;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += v;
-    }
-    const int excl = incl - cnt;
-    const int total = __shfl_sync(0xffffffffu, incl, 31);
-    for (int base = 0; base < total; base += 32) {
-        for (int i = max(excl, base); i < min(incl, base + 32); ++i)
-            owner[i - base] = (signed char)lane;
-        __syncwarp();
-        const int item = base + lane;
-        const bool valid = item < total;
-        const int o = valid ? (int)owner[lane] : 0;
-        __syncwarp();
-        SlabIdLor m;
-        m.k_lo = __shfl_sync(0xffffffffu, c.k_lo, o);
-        const int k = m.k_lo + item - __shfl_sync(0xffffffffu, excl, o);
-        const int to = __shfl_sync(0xffffffffu, t, o);
-        if constexpr (kBand) {
-            m.s_lo = __shfl_sync(0xffffffffu, c.s_lo, o);
-            m.s_hi = __shfl_sync(0xffffffffu, c.s_hi, o);
-            m.f0 = __shfl_sync(0xffffffffu, c.f0, o);
-            m.row0 = __shfl_sync(0xffffffffu, c.row0, o);
-            m.drow = __shfl_sync(0xffffffffu, c.drow, o);
-            m.reach = __shfl_sync(0xffffffffu, c.reach, o);
-        }
-        if (valid) range_slab_ids<kBand>(p, sp, m, k, [&](int id) { g(id, to); });
-    }
-}
-
 // atomicAdd(&counter[id], 1) for the calling lane, with one shared-memory update per
 // distinct id among the warp's active lanes (neighbouring LORs mostly share slabs). Returns
 // the lane's slot: the counter's old value plus its rank among the lanes with that id.
@@ -1021,18 +982,13 @@ __device__ __forceinline__ int warp_increment(int *counter, int id) {
     return first + __popc(peers & ((1u << lane) - 1u));
 }
 
-// Counting. Map calls over row-band slabs spread the (LOR, slice range) items of a warp
-// over its lanes (warp_slab_ids): their LORs span the whole field of view (tens of ranges
-// each, in numbers that differ between lanes, with a band computation per range), and
-// generated LORs of another axis group drop out here, idling their lanes in a loop per
-// lane (generated random pairs at 256 x 256 x 128: 239 against 264 ms per 50M, tensor
-// pairs 217 against 220 ms). Elsewhere a loop per lane measured faster: 1.4 % on the
-// 128 x 128 x 64 combined call, 4 % on the 128 x 128 x 64 map, where a range costs one
-// shared add.
+// Counting, one LOR per lane. (Spreading a warp's (LOR, slice range) items over its lanes,
+// which paid for maps over row bands while a range cost four conversions, now costs more in
+// shuffles than idle lanes do: 3M generated pairs at 256 x 256 x 128 counted in 1.33 ms with
+// it, 0.74 without.)
 template <int OP, bool kBand>
 __global__ void __launch_bounds__(kSegThreads) seg_count_kernel(const TorParams p, SegPlan sp) {
     extern __shared__ int hist[];  // [n_slabs]
-    __shared__ signed char owner_tab[kSegThreads / 32][32];
     for (int k = threadIdx.x; k < sp.n_slabs; k += kSegThreads) hist[k] = 0;
     if (blockIdx.x == 0 && threadIdx.x == 0) *sp.scanned = 0;
     __syncthreads();
@@ -1071,10 +1027,7 @@ __global__ void __launch_bounds__(kSegThreads) seg_count_kernel(const TorParams 
             }
             sp.range[t] = packed;
         }
-        if (OP == kMap && kBand) {
-            warp_slab_ids<kBand>(p, sp, owner_tab[threadIdx.x >> 5], ok, (int)t, c,
-                                 [&](int id, int) { atomicAdd(&hist[id], 1); });
-        } else if (ok) {
+        if (ok) {
             for (int k = c.k_lo; k <= c.k_hi; k++)
                 range_slab_ids<kBand>(p, sp, c, k, [&](int id) { atomicAdd(&hist[id], 1); });
         }
@@ -1183,7 +1136,10 @@ __global__ void __launch_bounds__(kSegThreads) seg_fill_kernel(const TorParams p
             slab_id_lor(p, sp, t, k_lo, k_hi, s_lo, s_hi, y1, z1, d1, dz, byv);
         for (int k = k_lo; k <= k_hi; k++)
             range_slab_ids<kBand>(p, sp, c, k, [&](int id) {
-                const int pos = warp_increment(cursor, id);
+                // Whole slices: a warp's LORs share their few ids (one shared add for all: 163
+                // against 352 us per 10M events). Bands: they spread over many (an add per
+                // lane: 0.69 against 1.07 ms for 3M generated pairs at 256 x 256 x 128).
+                const int pos = kBand ? atomicAdd(cursor + id, 1) : warp_increment(cursor, id);
                 sp.seg[tile_base[id] + pos] = (int)t;
             });
     }
@@ -1828,7 +1784,7 @@ bool slab_geometry(const TorParams &p, int pad, SegPlan &sp) {
         sp.nsl = want > 0 ? want : full;
         sp.band_rows = p.gy;
     } else {
-        int n = std::min(want > 0 ? want : kMinSlabSlices, p.gz);
+        int n = std::min({want > 0 ? want : kMinSlabSlices, p.gz, kMaxSlabSlices});
         sp.band_rows = 0;
         for (; n >= 1; n--) {
             int rows = std::min(p.gy, (int)((budget / n) / (size_t)slab_row_stride(p.gx, pad)));
