@@ -125,8 +125,9 @@ def _lors_of(d):
 
 # Images below this take torch's transposes: there a call's host time is what counts, and
 # ops.permuted_sum's is the longer one (2k-event step at 64 x 64 x 32: 131 us with torch's, 170
-# with it; from 2^20 voxels on its kernel is the faster by 20 us per step).
-_ONE_PASS_VOXELS = 1 << 18
+# with it; 60k-event projection at 101 x 93 x 47: 86 and 116 us). From 2^20 voxels on its kernel
+# saves more (400k-event back-projection at 128 x 128 x 64: 532 and 495 us).
+_ONE_PASS_VOXELS = 1 << 20
 
 
 def _kernel_view(model, image, axis):
