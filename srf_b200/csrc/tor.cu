@@ -117,7 +117,6 @@ struct TorParams {
     float *proj_out;
     int *count_out;   // kCount: [n] voxels with non-zero weight, [n] window voxels visited
     int use_slab;     // slab kernels: never (0), where they apply (1), by few_lors (2)
-    float left;       // scatter ops: the weight a LOR leaves in a slice, about
     float box_x0, box_y0;  // -bound / inter - 1/2: voxel-centre units of a coordinate 0
     PairConsts pc;    // the geometry as operands of the paired arithmetic (slab kernels)
     float fit;        // largest box half-extent that no window clips (box_in_window)
@@ -675,9 +674,8 @@ __device__ __forceinline__ void seg_lor(const LorRec *rec, int64_t t, SegLor &L)
     L.inv_dz = __frcp_rn(L.dz);
 }
 
-// The op's factor of LOR t's weights (lor_value_scale) in L: a scatter op's magnitude as
-// log2 in kE and by itself in L.scale with its sign, the projection's in L.scale. False
-// when the LOR contributes nothing.
+// The op's factor of LOR t's weights (lor_value_scale) in L: the back-projection's as log2 in
+// kE, the others' in L.scale. False when the LOR contributes nothing.
 template <int OP>
 __device__ __forceinline__ bool seg_value(const TorParams &p, int64_t t, SegLor &L) {
     LorConst c;
@@ -687,10 +685,8 @@ __device__ __forceinline__ bool seg_value(const TorParams &p, int64_t t, SegLor 
     if (!lor_value_scale<OP>(p, t, c)) return false;
     L.scale = c.scale;
     L.general = L.general || c.all || !(fabsf(c.scale) <= 3.0e38f);
-    if (OP != kProj) {
-        if (!(fabsf(c.scale) > 0.0f)) return L.general && c.scale != 0.0f;  // 0 adds nothing
-        L.kE += OP == kBack ? c.k0s : log2_abs(c.scale);
-    }
+    if (OP != kProj && c.scale == 0.0f) return L.general;  // finite weights times 0
+    if (OP == kBack) L.kE += c.k0s;
     return true;
 }
 
@@ -862,11 +858,12 @@ constexpr int kSegThreads = 512;
 constexpr int kSegItems = 8;
 constexpr int kSegTile = kSegThreads * kSegItems;
 constexpr int kMaxSlabs = 4096;
-// Threads of a slab CTA (one CTA per SM): 72 registers each, the fewest that spill little in
-// the voxel loops. 640 / 768 / 896 / 1024 threads took 5.17 / 5.06 / 5.07 / 5.80 ms (projection)
-// and 7.09 / 6.94 / 6.77 / 7.27 ms (back-projection) for 10M events at 128 x 128 x 64.
+// Threads of a slab CTA (one CTA per SM). 640 / 768 / 896 / 1024 threads took 5.17 / 5.06 /
+// 5.07 / 5.80 ms (projection: 72 registers are the fewest that spill little in the voxel loops)
+// and 12.26 / 11.15 / 10.66 / 10.47 ms (back-projection: it waits for its shared-memory adds)
+// for 10M events at 128 x 128 x 64; the map of 6M pairs there 9.73 / 9.05 / 8.41 / 8.08 ms.
 constexpr int kProjThreads = 896;
-constexpr int kScatThreads = 896;
+constexpr int kScatThreads = 1024;
 constexpr int slab_threads(int op) { return op == kProj ? kProjThreads : kScatThreads; }
 constexpr size_t kSlabSmemBytes = 220 * 1024;  // of the 227 KB a CTA can opt into
 constexpr int kMaxSlabSlices = 1024;           // entries of the slab's table of slice planes
@@ -1194,15 +1191,6 @@ struct SliceBox {
     bool in;
 };
 
-// How a walk uses its weights: gathers w * slab (projection), adds them to a float slab, or
-// adds them to a fixed-point slab (kWide: weights of 2^shift units and more).
-enum WalkMode { kGather = 0, kFloat = 1, kFixed = 2, kWide = 3 };
-
-// 2^-149, the spacing of subnormal floats: w * kSubnormal has the integer nearest to w as
-// its bits for 0 <= w < 2^24 (one product in place of a conversion).
-constexpr float kSubnormal = 1.401298464324817e-45f;
-constexpr int kFixedBits = 24;
-
 // The crossing (tor.cu.cc:22-48) of slice s (counted from the slab's first) and the first
 // column and row of the H x W box that is walked there.
 //
@@ -1242,8 +1230,7 @@ __device__ __forceinline__ SliceBox slice_box(const TorParams &p, const SlabView
 
 // The slices a .. a + cnt - 1 (counted from the slab's first) of the lane's segment; the
 // warp's lanes walk n_max slices together, H rows and W columns of each (at least every
-// lane's own box). kGather returns the sum of w * slab in acc; kFixed / kWide add the units
-// they put into the slab to `units`.
+// lane's own box). Projection: returns the sum of w * slab. Scatter ops: adds the weights.
 //
 // These kernels are bound by instruction issue and FP32 throughput (the earlier form issued
 // on 86 % of the cycles): of ~420 lane-instructions per (LOR, slice) only ~125 were the
@@ -1253,14 +1240,18 @@ __device__ __forceinline__ SliceBox slice_box(const TorParams &p, const SlabView
 // half-extent b holds at most floor(2 b) + 1 voxel centres) instead of reduced over the warp
 // in every slice, and the window is left out where it decides nothing. Two slices go side
 // by side through columns, rows and voxels, two floats per instruction (halving the loops'
-// own cost; one slice at a time measured 5.25 and 7.77 ms against 5.07 and 6.77 for the
-// projection and back-projection of 10M events); a slice that is not crossed follows its
-// neighbour with a cut-off nothing passes. Rows outside the slab's rows lie in its padding,
-// which reads 0 and is never flushed.
-template <int OP, int P, int W, int MODE, bool kWindow>
-__device__ __forceinline__ void walk_segment(const TorParams &p, const SlabView &v,
-                                             const SegLor &L, int a, int cnt, int n_max, int H,
-                                             int shift, float &acc, unsigned long long &units) {
+// own cost; one slice at a time measured 5.25 ms against 5.07 for the projection of 10M
+// events); a slice that is not crossed follows its neighbour with a cut-off nothing
+// passes. Rows outside the slab's rows lie in its padding, which reads 0 and is never flushed.
+//
+// A scatter op adds floats in shared memory, a loop of a load and a compare-and-swap. (32-bit
+// integer adds took 6.5 ms where these take 10.5 for 10M events, but hold a weight in 20 bits
+// of the typical one: voxels that only tails reach lost digits or everything, and factors
+// above 1, where TOF is sharper than the tube, have no place in the word.)
+template <int OP, int P, int W, bool kWindow>
+__device__ __forceinline__ float walk_segment(const TorParams &p, const SlabView &v,
+                                              const SegLor &L, int a, int cnt, int n_max,
+                                              int H) {
     const float lo_x = p.box_x0 - L.bxv, lo_y = p.box_y0 - L.byv;
     const F2 ux2 = both(L.ux), uy2 = both(L.uy), k1 = both(L.k1);
     float acc0 = 0.0f, acc1 = 0.0f;
@@ -1287,7 +1278,6 @@ __device__ __forceinline__ void walk_segment(const TorParams &p, const SlabView 
             }
             const F2 cy = pack2(b0.cy, b1.cy);
             F2 yc = pack2((b0.ym - kMagic) + 0.5f, (b1.ym - kMagic) + 0.5f);  // exact
-            unsigned put = 0;  // < 2 * 64 * 2^24
 #pragma unroll 1
             for (int j = 0; j < H; j++) {
                 const F2 dy = sub2(cy, fma2(p.pc.iy, yc, p.pc.bb));
@@ -1302,31 +1292,23 @@ __device__ __forceinline__ void walk_segment(const TorParams &p, const SlabView 
                     unpack2(d2, d0, d1);
                     unpack2(ex, e0, e1);
                     const float w0 = fast_exp2(e0), w1 = fast_exp2(e1);
-                    if (MODE == kGather) {
+                    if (OP == kProj) {
                         if (d0 < n0) acc0 = fmaf(w0, r0[c], acc0);
                         if (d1 < n1) acc1 = fmaf(w1, r1[c], acc1);
-                    } else if (MODE == kFloat) {
-                        if (d0 < n0) atomicAdd(r0 + c, L.scale < 0.0f ? -w0 : w0);
-                        if (d1 < n1) atomicAdd(r1 + c, L.scale < 0.0f ? -w1 : w1);
                     } else {
-                        const unsigned u0 = d0 < n0 ? __float_as_uint(w0 * kSubnormal) : 0u;
-                        const unsigned u1 = d1 < n1 ? __float_as_uint(w1 * kSubnormal) : 0u;
-                        put += u0 + u1;
-                        atomicAdd(reinterpret_cast<unsigned *>(r0) + c,
-                                  MODE == kWide ? u0 << shift : u0);
-                        atomicAdd(reinterpret_cast<unsigned *>(r1) + c,
-                                  MODE == kWide ? u1 << shift : u1);
+                        // back-projection: the scale is in w's exponent already
+                        if (d0 < n0) atomicAdd(r0 + c, OP == kBack ? w0 : w0 * L.scale);
+                        if (d1 < n1) atomicAdd(r1 + c, OP == kBack ? w1 : w1 * L.scale);
                     }
                 }
                 r0 += v.rs;
                 r1 += v.rs;
                 yc = add2(yc, p.pc.one);
             }
-            if (MODE == kFixed || MODE == kWide) units += (unsigned long long)put << shift;
         }
         __syncwarp();
     }
-    acc = acc0 + acc1;
+    return acc0 + acc1;
 }
 
 // A segment whose LOR takes the general walk (a map LOR with a zero or non-finite divisor,
@@ -1352,136 +1334,27 @@ __device__ __noinline__ void general_segment(const TorParams &p, int64_t t, int 
     if (OP == kProj) atomicAdd(p.proj_out + t, acc * L.scale);
 }
 
-// Fixed-point slabs (scatter ops). A float add in shared memory is a loop of a load and a
-// compare-and-swap; an integer add is one instruction (measured 2.5e12 against 8.3e11 adds
-// per second at hashed addresses). A slab pass therefore adds its weights as integers of
-// a unit 2^(E - bits), E the mean exponent of its LORs' scales (over a sample) and bits 20,
-// or 21 where a voxel gets few adds. With n typical adds a voxel's sum is ~0.35 n 2^20
-// units, its rounding error 0.29 sqrt(n): 8e-8 relative at n = 100, as float adds leave.
-// Scales from 2^-4 to 2^10 times the typical one go in (the large ones through kWide's
-// shift); the few LORs outside take general_segment, and where the sample has more of them
-// than 1 in 32, or of the other sign, the pass adds floats. So it does with fewer than
-// kMinFullAdds full weights per voxel (no gain, and nothing to average over) and for tubes
-// that leave less than one full weight per slice, whose scales have no typical size.
-// Against float adds (measured, 128 x 128 x 64): back-projection of 10M events 11.41 ->
-// 6.54 ms, adjoint of 1M 1.36 -> 0.88 ms, map of 6M pairs 8.6 -> 5.6 ms; 50k-LOR subsets equal.
-// Nothing is lost to a wrap: every lane also sums the units it adds in 64 bits, and the pass
-// is flushed only if the slab's words sum to the same. Otherwise it is redone over a shorter
-// stretch of the list, below kMinPass segments with float adds.
-constexpr int kMinBits = 20, kMaxBits = 21;  // of a typical LOR's full weight
-constexpr int kBelowBits = 4;
-constexpr int kWideBits = 7;
-constexpr int kMinPass = 1024;
-constexpr float kMeanFullAdds = 128.0f;  // longest pass: full weights per voxel
-constexpr float kMinFullAdds = 0.5f;     // shortest one in fixed point
-constexpr float kMinLeft = 1.0f;
-
-// Exponent of a scale's magnitude (subnormals count as 2^-127).
-__device__ __forceinline__ int scale_exponent(float s) {
-    return (int)((__float_as_uint(s) >> 23) & 0xffu) - 127;
-}
-
-struct PassPlan {
-    int fixed;     // 1: fixed point
-    int exponent;  // of the typical scale
-    int bits;      // of its full weight in units
-    int negative;  // sign of the scales
-};
-
-// What a CTA's threads share about the slab pass at hand: read where it is needed rather
-// than held in the registers that the voxel loops want.
-struct Pass {
-    const int *seg;  // its segments
-    int n_seg;
-    int S0, S1;      // slices
-    int done;        // segments below had their general walk in an earlier try
-    int floats;      // add floats
-    PassPlan plan;
-    int64_t img0;    // frame's offset in the image
-};
-
-// The plan of a slab pass from a sample of its segments' scales (every thread takes one).
-template <int OP>
-__device__ __forceinline__ PassPlan plan_pass(const TorParams &p, const int *seg, int n_seg,
-                                              float full_adds, int *stat) {
-    const int lane = threadIdx.x & 31;
-    PassPlan plan;
-    plan.exponent = plan.negative = 0;
-    plan.bits = min(kMaxBits, max(kMinBits, 24 - (int)ceilf(__log2f(full_adds))));
-    plan.fixed = 0;
-    if (p.left < kMinLeft || full_adds < kMinFullAdds) return plan;
-    if (OP == kMap && !p.values) {  // generated LORs: every scale is 1
-        plan.fixed = 1;
-        plan.exponent = 0;
-        plan.negative = 0;
-        return plan;
-    }
-    LorConst c;
-    c.scale = 0.0f;
-    bool use = false;
-    {
-        const int64_t at = (int64_t)n_seg * threadIdx.x / blockDim.x;
-        c.all = false;
-        use = lor_value_scale<OP>(p, seg[at], c) && !c.all && fabsf(c.scale) > 0.0f &&
-              fabsf(c.scale) < 3.0e38f;
-    }
-    const int ex = scale_exponent(c.scale);
-    if (threadIdx.x < 4) stat[threadIdx.x] = 0;
-    __syncthreads();
-    const int n = __popc(__ballot_sync(0xffffffffu, use));
-    const int neg = __popc(__ballot_sync(0xffffffffu, use && c.scale < 0.0f));
-    const int sum = __reduce_add_sync(0xffffffffu, use ? ex : 0);
-    if (lane == 0) {
-        atomicAdd(stat, n);
-        atomicAdd(stat + 1, neg);
-        atomicAdd(stat + 2, sum);
-    }
-    __syncthreads();
-    const int total = stat[0];
-    plan.negative = 2 * stat[1] > total;
-    plan.exponent = total ? (int)rintf((float)stat[2] / (float)total) : 0;
-    const bool odd = use && ((c.scale < 0.0f) != (plan.negative != 0) ||
-                             ex < plan.exponent - kBelowBits ||
-                             ex >= plan.exponent + kFixedBits - plan.bits + kWideBits);
-    const int n_odd = __popc(__ballot_sync(0xffffffffu, odd));
-    if (lane == 0) atomicAdd(stat + 3, n_odd);
-    __syncthreads();
-    plan.fixed = total > 0 && 32 * stat[3] <= total &&
-                 plan.exponent > -90 && plan.exponent < 90;
-    __syncthreads();
-    return plan;
-}
-
-// The segments of a slab pass, one per lane.
+// The segments seg[0, n_seg) of a slab of slices [S0, S1), one per lane.
 template <int OP, int P>
 __device__ __forceinline__ void walk_segments(const TorParams &p, const SegPlan &sp,
-                                              const SlabView &v, const volatile Pass &ps,
-                                              unsigned long long &units) {
+                                              const SlabView &v, const int *seg, int n_seg,
+                                              int S0, int S1, int64_t img0) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     constexpr int kStep = slab_threads(OP);
-    for (int q0 = warp * 32; q0 < ps.n_seg; q0 += kStep) {
+    for (int q0 = warp * 32; q0 < n_seg; q0 += kStep) {
         SegLor L;
         L.bxv = L.byv = 0.0f;
-        int a = 0, cnt = 0, w = 1, h = 1, shift = 0;
+        int a = 0, cnt = 0, w = 1, h = 1;
         int t = -1;
         const int q = q0 + lane;
-        if (q < ps.n_seg) {
-            t = __ldg(ps.seg + q);
-            if (q + kStep < ps.n_seg) {  // the next round's record on its way to L2
-                const int u = __ldg(ps.seg + q + kStep);
+        if (q < n_seg) {
+            t = __ldg(seg + q);
+            if (q + kStep < n_seg) {  // the next round's record on its way to L2
+                const int u = __ldg(seg + q + kStep);
                 asm volatile("prefetch.global.L2 [%0];" :: "l"(sp.rec + u));
             }
             seg_lor(sp.rec, t, L);
             if (seg_value<OP>(p, t, L)) {
-                const int S0 = ps.S0, S1 = ps.S1;
-                if (OP != kProj && ps.plan.fixed) {
-                    const int ex = scale_exponent(L.scale) - ps.plan.exponent;
-                    const int over = ex - (kFixedBits - ps.plan.bits);
-                    L.general = L.general || (L.scale < 0.0f) != (ps.plan.negative != 0) ||
-                                ex < -kBelowBits || over >= kWideBits;
-                    shift = max(0, over + 1);
-                    if (!ps.floats) L.kE += (float)(ps.plan.bits - ps.plan.exponent - shift);
-                }
                 if (!L.general) {
                     a = max(L.s_lo, S0);
                     cnt = max(0, min(L.s_hi, S1 - 1) - a + 1);
@@ -1489,8 +1362,8 @@ __device__ __forceinline__ void walk_segments(const TorParams &p, const SegPlan 
                     // columns and rows of its largest box (voxel centres within b)
                     w = 1 + (int)fminf(2.0f * L.bxv, (float)(P - 1));
                     h = 1 + (int)fminf(2.0f * L.byv, (float)(P - 1));
-                } else if (q >= ps.done) {
-                    general_segment<OP, P>(p, t, S0, S1, v.R0, v.R1, ps.img0);
+                } else {
+                    general_segment<OP, P>(p, t, S0, S1, v.R0, v.R1, img0);
                 }
             }
         }
@@ -1501,27 +1374,13 @@ __device__ __forceinline__ void walk_segments(const TorParams &p, const SegPlan 
         const bool clipped = __any_sync(
             0xffffffffu, cnt > 0 && !(L.bxv < p.fit && L.byv < p.fit));
         float acc = 0.0f;
-        auto walk = [&](auto mode) {
-            constexpr int kMode = decltype(mode)::value;
-            if (clipped)
-                walk_segment<OP, P, P, kMode, true>(p, v, L, a, cnt, n_max, P, shift, acc, units);
-            else
-                with_width<P>(w, [&](auto W) {
-                    walk_segment<OP, P, decltype(W)::value, kMode, false>(
-                        p, v, L, a, cnt, n_max, h, shift, acc, units);
-                });
-        };
-        if constexpr (OP == kProj) {
-            walk(std::integral_constant<int, kGather>{});
-            if (cnt > 0) atomicAdd(p.proj_out + t, acc * L.scale);
-        } else {
-            if (ps.floats)
-                walk(std::integral_constant<int, kFloat>{});
-            else if (__any_sync(0xffffffffu, cnt > 0 && shift > 0))
-                walk(std::integral_constant<int, kWide>{});
-            else
-                walk(std::integral_constant<int, kFixed>{});
-        }
+        if (clipped)
+            acc = walk_segment<OP, P, P, true>(p, v, L, a, cnt, n_max, P);
+        else
+            with_width<P>(w, [&](auto W) {
+                acc = walk_segment<OP, P, decltype(W)::value, false>(p, v, L, a, cnt, n_max, h);
+            });
+        if (OP == kProj && cnt > 0) atomicAdd(p.proj_out + t, acc * L.scale);
     }
 }
 
@@ -1533,16 +1392,13 @@ __device__ __forceinline__ void clear_slab(float *slab, int n) {
 }
 
 // Persistent pass over the slab-major segment list (all TOR ops but the count). Scatter
-// ops accumulate into the slab with shared atomics and flush once per slab pass; the
+// ops accumulate into the slab with shared atomics and flush once per slab; the
 // projection gathers from the slab (loaded from the image) and adds each LOR's partial
 // sum to its output. One segment per lane.
 template <int OP, int P>
 __global__ void __launch_bounds__(slab_threads(OP), 1)
 tor_slab_kernel(const __grid_constant__ TorParams p, const __grid_constant__ SegPlan sp) {
     extern __shared__ float smem[];
-    __shared__ int stat[4];
-    __shared__ unsigned long long sums[2];
-    __shared__ Pass pass;
     float *const zs = smem;  // [nsl] planes of the slab's slices
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     constexpr int kThreads = slab_threads(OP);
@@ -1602,77 +1458,28 @@ tor_slab_kernel(const __grid_constant__ TorParams p, const __grid_constant__ Seg
                 for (int ix = lane; ix < p.gx; ix += 32)
                     d[ix] = iy < nbr ? __ldg(g + (int64_t)ix * p.sx) : 0.0f;
             }
-            if (threadIdx.x == 0) pass = Pass{seg, n_seg, S0, S1, 0, 1, PassPlan{}, img0};
-            __syncthreads();
-            unsigned long long none = 0;
-            walk_segments<OP, P>(p, sp, v, pass, none);
-            __syncthreads();
         } else {
-            const float per_voxel = p.left / ((float)p.gx * (float)nbr);
-            const int longest = (int)fminf(kMeanFullAdds / per_voxel, 1.0e9f);
-            int len = max(kMinPass, longest);
-            const PassPlan plan =
-                plan_pass<OP>(p, seg, n_seg, per_voxel * (float)min(len, n_seg), stat);
-            const int n = slab_floats(S1 - S0, p.gx, sp.band_rows, pad);
-            int at = 0, tried = 0;  // flushed up to `at`; general walks done up to `tried`
-            bool floats = !plan.fixed;
-            while (at < n_seg) {
-                const int m = floats ? n_seg - at : min(len, n_seg - at);
-                clear_slab<kThreads>(slab, n);
-                if (threadIdx.x < 2) sums[threadIdx.x] = 0;
-                if (threadIdx.x == 0)
-                    pass = Pass{seg + at, m, S0, S1, tried - at, floats, plan, img0};
-                __syncthreads();
-                unsigned long long units = 0;
-                walk_segments<OP, P>(p, sp, v, pass, units);
-                tried = max(tried, at + m);
-                __syncthreads();
-                if (!floats) {  // the units added against the words' sum
-                    unsigned long long words = 0;
-                    for (int i = threadIdx.x; i < (n + 3) / 4; i += kThreads) {
-                        const uint4 q = reinterpret_cast<const uint4 *>(slab)[i];
-                        words += (unsigned long long)q.x + q.y;
-                        words += (unsigned long long)q.z + q.w;
-                    }
+            clear_slab<kThreads>(slab, slab_floats(S1 - S0, p.gx, sp.band_rows, pad));
+        }
+        __syncthreads();
+        walk_segments<OP, P>(p, sp, v, seg, n_seg, S0, S1, img0);
+        __syncthreads();
+        if (OP != kProj) {
+            float *out = p.image_out + img0 + (int64_t)S0 * p.sz + (int64_t)R0 * p.sy;
+            for (int r = warp; r < (S1 - S0) * nbr; r += kThreads / 32) {
+                const int sl = r / nbr, iy = r - sl * nbr;
+                const float *src = slab + origin + sl * ss + iy * rs;
+                float *g = out + (int64_t)sl * p.sz + (int64_t)iy * p.sy;
+                for (int ix = lane; ix < p.gx; ix += 128) {
 #pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) {
-                        units += __shfl_xor_sync(0xffffffffu, units, o);
-                        words += __shfl_xor_sync(0xffffffffu, words, o);
-                    }
-                    if (lane == 0) {
-                        atomicAdd(&sums[0], units);
-                        atomicAdd(&sums[1], words);
-                    }
-                    __syncthreads();
-                    const bool wrapped = sums[0] != sums[1];
-                    __syncthreads();
-                    if (wrapped) {
-                        len = m / 4;
-                        floats = len < kMinPass;
-                        continue;
+                    for (int u = 0; u < 4; u++) {
+                        const int c = ix + 32 * u;
+                        const float val = c < p.gx ? src[c] : 0.0f;
+                        if (val != 0.0f) atomicAdd(g + (int64_t)c * p.sx, val);
                     }
                 }
-                const float size = exp2f((float)(plan.exponent - plan.bits));
-                const float unit = plan.negative ? -size : size;
-                float *out = p.image_out + img0 + (int64_t)S0 * p.sz + (int64_t)R0 * p.sy;
-                for (int r = warp; r < (S1 - S0) * nbr; r += kThreads / 32) {
-                    const int sl = r / nbr, iy = r - sl * nbr;
-                    const float *src = slab + origin + sl * ss + iy * rs;
-                    float *g = out + (int64_t)sl * p.sz + (int64_t)iy * p.sy;
-                    for (int ix = lane; ix < p.gx; ix += 128) {
-#pragma unroll
-                        for (int u = 0; u < 4; u++) {
-                            const int c = ix + 32 * u;
-                            const float word = c < p.gx ? src[c] : 0.0f;
-                            const float val =
-                                floats ? word : unit * (float)__float_as_uint(word);
-                            if (val != 0.0f) atomicAdd(g + (int64_t)c * p.sx, val);
-                        }
-                    }
-                }
-                at += m;
-                __syncthreads();
             }
+            __syncthreads();
         }
         pos = end;
     }
@@ -1730,8 +1537,6 @@ int tor_setup(TorParams &p, const int *grid, const float *center, const float *s
     // ~1e-6 (patch * inter)^2 of the exact value, the margin is 2^-16 (patch * inter)^2.
     const float span = (float)p.patch * std::max(p.inter_x, p.inter_y);
     p.box_e = span * span * (1.0f / 65536.0f);
-    // 2 pi sigma^2 over the voxel area, 1.4 for oblique LORs
-    p.left = std::max(1.0e-3f, 1.4f * 6.2832f * p.tor_sigma2 / (p.inter_x * p.inter_y));
     p.box_x0 = -p.l_bound * p.inv_x - 0.5f;
     p.box_y0 = -p.b_bound * p.inv_y - 0.5f;
     p.fit = std::min((float)p.half + 0.5f, (float)(p.patch - p.half) - 0.5f) - 1.0f / 1024.0f;
