@@ -607,7 +607,7 @@ __device__ __forceinline__ bool prepare_any(const TorParams &p, int64_t t, LorCo
 //
 // General walk: LORs at more than ~83 degrees from the slice axis (A > kMaxSlope2; a
 // dominant-axis group's have A <= 3), where the vertex form loses digits and few slices
-// are crossed anyway.
+// are crossed anyway, and LORs whose TOF terms are not finite.
 struct __align__(16) LorRec {
     float4 a, b, c, d;
 };
@@ -632,7 +632,10 @@ __device__ __forceinline__ LorRec make_rec(const TorParams &p, const LorConst &L
         // |C - X|^2 = A (h - h0)^2 + E at h = 0
         kE = (float)(-(double)p.a_coef * (ex * ex + ey * ey - A * h0 * h0));
     }
-    const int general = slope2 <= kMaxSlope2 ? 0 : 1 << (2 * kSliceBits);
+    // a TOF term beyond the floats (a centre at infinity: the weight is 0, but the vertex form
+    // has inf - inf) also takes the general walk
+    const bool plain = slope2 <= kMaxSlope2 && fabsf(z0) + fabsf(kA) + fabsf(kE) <= 3.0e38f;
+    const int general = plain ? 0 : 1 << (2 * kSliceBits);
     LorRec r;
     r.a = make_float4(L.x1, L.y1, L.z1, L.d0);
     r.b = make_float4(L.d1, L.dz, L.ux, L.uy);
@@ -1312,7 +1315,7 @@ __device__ __forceinline__ float walk_segment(const TorParams &p, const SlabView
 }
 
 // A segment whose LOR takes the general walk (a map LOR with a zero or non-finite divisor,
-// a LOR far from the slice axis): its slices [S0, S1) and rows [R0, R1) straight on the
+// a LOR far from the slice axis or with a TOF centre that is not finite): its slices [S0, S1) and rows [R0, R1) straight on the
 // image in global memory.
 template <int OP, int P>
 __device__ __noinline__ void general_segment(const TorParams &p, int64_t t, int S0, int S1,

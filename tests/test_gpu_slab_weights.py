@@ -1,6 +1,6 @@
 """Weights of the slab kernels over the range that a float holds: factors above 1 (TOF sharper
 than the tube), voxels that only the tails of the two Gaussians reach, TOF centres that are
-not numbers.
+not numbers or at infinity.
 
 Tolerances. The slab kernels and the oracle take the same float decisions; their weights
 differ by the exponent's error. A crossing point is off by up to 1.7e-5 mm here (the
@@ -135,3 +135,28 @@ def test_centre_that_is_not_a_number(many):
         assert many or nan.sum() == 1
         assert torch.equal(torch.isnan(got), nan)
         assert K.rel_l2(got[~nan].cpu().numpy(), ref[~nan].cpu().numpy()) <= 1e-5
+
+
+@pytest.mark.parametrize("row", [6, 7, 8])
+@pytest.mark.parametrize("value", [np.inf, -np.inf, 1e30])
+def test_centre_at_infinity(row, value):
+    """A LOR whose TOF centre is infinitely far away weighs nothing anywhere (tolerance for the
+    rest as above)."""
+    n, voxel, kw, tof = 60_000, 3.2, 10.19, (6.0, 1139.77)
+    size = [g * voxel for g in GRID]
+    lors = _lors(n, 13)
+    away = np.arange(50) * 1100
+    lors[row, away] = value
+    rest = np.delete(lors, away, axis=1)
+    L, V = _cu(lors), torch.full((n,), 2.0, device="cuda")
+    img = torch.rand(GRID[::-1], device="cuda") + 0.1
+    a = (GRID, CENTER, size, kw, False, *tof)
+    pv = ops.tor_projection(L, img, *a, layout="cn").cpu().numpy()
+    assert not pv[away].any()
+    ref = O.tor_projection(rest, img.cpu().numpy(), *a, mode="f32", contract=True)
+    assert K.rel_l2(np.delete(pv, away), ref) <= 1e-5
+    ref = O.tor_backprojection(rest, np.full(rest.shape[1], 2.0, np.float32), *a, mode="f32",
+                               contract=True)
+    for got in (ops.tor_backprojection(img, L, V, *a, layout="cn"),
+                ops.tor_backproject_adjoint(0.25 * V, L, *a, layout="cn")):
+        assert K.rel_l2(got.cpu().numpy(), ref) <= 1e-5
