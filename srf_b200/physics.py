@@ -141,13 +141,11 @@ def _kernel_view(model, image, axis):
 
 
 def _kernel_image(model, image, axis):
-    """``model.kernel_geometry(image, axis)``, the copy by ``ops.permuted_sum`` where it
-    takes the image."""
-    if type(model) is not SplitLoRsModel or image.data.numel() < _ONE_PASS_VOXELS \
-            or not ops.permutable(image.data):
+    """``model.kernel_geometry(image, axis)``, a copy that is needed by ``permuted_sum``."""
+    if type(model) is not SplitLoRsModel:
         return model.kernel_geometry(image, axis)
     view, g, c, s = _kernel_view(model, image, axis)
-    return ops.permuted_sum([view]), g, c, s
+    return permuted_sum([view]), g, c, s
 
 
 def projection(model, image, data):
@@ -174,10 +172,15 @@ def projection(model, image, data):
 
 
 def permuted_sum(views):
-    """The sum of permuted views as a contiguous tensor: ``ops.permuted_sum`` where it takes
-    them (dense CUDA float32 stacks), else torch operations in the same order."""
+    """The sum of permuted views as a contiguous tensor (one contiguous view is that view):
+    ``ops.permuted_sum`` where it takes them (dense CUDA float32 stacks), else torch
+    operations in the same order."""
+    if len(views) == 1 and views[0].is_contiguous():
+        return views[0]
     if views[0].numel() >= _ONE_PASS_VOXELS and all(ops.permutable(v) for v in views):
         return ops.permuted_sum(views)
+    if len(views) == 1:
+        return views[0].contiguous()
     out = views[0].clone()
     for v in views[1:]:
         out = out.add_(v)
