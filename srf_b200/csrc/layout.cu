@@ -78,7 +78,7 @@ extern "C" int srf_permute_sum(float *out, const int *dims, int64_t n_frames, in
     PermuteArgs a{};
     a.out = out;
     a.n_src = n_sources;
-    int64_t blocks = n_frames;
+    int64_t blocks = 1;
     a.frame = 1;
     for (int k = 0; k < 3; k++) {
         if (dims[k] < 0) return SRF_ERR_INVALID_ARGUMENT;
@@ -86,10 +86,11 @@ extern "C" int srf_permute_sum(float *out, const int *dims, int64_t n_frames, in
         a.tiles[k] = (dims[k] + kSide - 1) / kSide;
         a.frame *= dims[k];
         if (a.frame > ((int64_t)1 << 31) - 1) return SRF_ERR_UNSUPPORTED;
-        blocks *= a.tiles[k];
+        blocks *= a.tiles[k];  // at most 2^31: tiles <= dims
     }
-    if (blocks == 0) return SRF_OK;
-    if (blocks > INT32_MAX) return SRF_ERR_UNSUPPORTED;
+    if (blocks == 0 || n_frames == 0) return SRF_OK;
+    if (n_frames > INT32_MAX / blocks) return SRF_ERR_UNSUPPORTED;
+    blocks *= n_frames;
     if (!out) return SRF_ERR_INVALID_ARGUMENT;
     for (int s = 0; s < n_sources; s++) {
         if (!sources[s] || sources[s] == out) return SRF_ERR_INVALID_ARGUMENT;
@@ -98,7 +99,8 @@ extern "C" int srf_permute_sum(float *out, const int *dims, int64_t n_frames, in
         a.fast[s] = -1;
         for (int k = 0; k < 3; k++) {
             a.stride[s][k] = strides[3 * s + k];
-            if (a.stride[s][k] < 1) return SRF_ERR_INVALID_ARGUMENT;
+            // beyond the frame the sum below could pass it by overflowing
+            if (a.stride[s][k] < 1 || a.stride[s][k] > a.frame) return SRF_ERR_INVALID_ARGUMENT;
             if (a.stride[s][k] == 1 && (a.fast[s] < 0 || a.d[k] > a.d[a.fast[s]])) a.fast[s] = k;
         }
         int64_t last = 0;

@@ -1,9 +1,13 @@
-"""Axis-order changes below the size of the one-pass kernel: what torch is asked to copy."""
+"""Axis-order changes: what torch is asked to copy below the size of the one-pass kernel, and
+what that kernel's entry point refuses on the host."""
+
+import ctypes
 
 import pytest
 import torch
 from torch.utils._python_dispatch import TorchDispatchMode
 
+from srf_b200 import _lib
 from srf_b200.physics import permuted_sum
 
 COPIES = {"aten::clone", "aten::copy_", "aten::_to_copy"}
@@ -41,3 +45,24 @@ def test_several_views_add_in_order():
     out = permuted_sum(views)
     assert out.is_contiguous() and torch.equal(out, (a + b) + c)
     assert torch.equal(a, views[0])  # sources stay as they were
+
+
+def _call(dims, frames, strides, sources=(4096,), out=8192):
+    n = len(sources)
+    return _lib.load().srf_permute_sum(
+        ctypes.c_void_p(out), (ctypes.c_int * 3)(*dims), frames, n,
+        (ctypes.c_void_p * n)(*sources), (ctypes.c_int64 * len(strides))(*strides), None)
+
+
+def test_entry_point_refuses_before_any_launch():
+    """Strides that leave the frame, also where their sum passes 2^63, and counts of frames
+    that no launch holds (status 1 invalid argument, 3 unsupported)."""
+    assert _call((5, 4, 3), 1, (12, 3, 0)) == 1
+    assert _call((5, 4, 3), 1, (13, 3, 1)) == 1
+    assert _call((5, 4, 3), 1, (1 << 62, 3, 1)) == 1           # 4 * 2^62 = 0 mod 2^64
+    assert _call((5, 4, 3), 1, (1, 1 << 61, 1 << 62)) == 1     # 3 * 2^61 + 2 * 2^62 < 0
+    assert _call((5, 4, 3), 1, (12, 3, 1), (8192,)) == 1       # out among the sources
+    assert _call((64, 16, 16), 1 << 62, (256, 16, 1)) == 3     # 4 tiles * 2^62 = 0 mod 2^64
+    assert _call((16, 16, 16), 1 << 31, (256, 16, 1)) == 3
+    assert _call((5, 0, 3), 1 << 62, (3, 3, 1)) == 0           # nothing to do
+    assert _call((5, 4, 3), 0, (12, 3, 1)) == 0
