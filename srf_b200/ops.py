@@ -346,16 +346,19 @@ def mlem_update_(image, effinv, bp):
 
 def permutable(t):
     """Whether ``permuted_sum`` takes ``t``: float32 on a CUDA device, three axes (or frames
-    and three axes) of a dense stack in any axis order within its frames, no gradient."""
+    and three axes) of a dense stack in any axis order within its frames, no gradient, no
+    negation to be applied on reading, a size that one launch indexes."""
     if not (t.is_cuda and t.dtype == torch.float32 and t.dim() in (3, 4) and t.numel() > 0) \
-            or (t.requires_grad and torch.is_grad_enabled()):
+            or (t.requires_grad and torch.is_grad_enabled()) or t.is_neg():
         return False
-    dense = 1
+    dense = tiles = 1
     for st, n in sorted(zip(t.stride()[-3:], t.shape[-3:]), key=lambda a: (a[0], a[1])):
         if n > 1 and st != dense:
             return False
         dense *= n
-    return t.dim() == 3 or t.shape[0] == 1 or t.stride(0) == dense
+        tiles *= -(-n // 16)
+    frames = t.shape[0] if t.dim() == 4 else 1
+    return dense < 1 << 31 and tiles * frames < 1 << 31 and (frames == 1 or t.stride(0) == dense)
 
 
 def permuted_sum(views):

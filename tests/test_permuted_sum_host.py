@@ -7,7 +7,7 @@ import pytest
 import torch
 from torch.utils._python_dispatch import TorchDispatchMode
 
-from srf_b200 import _lib
+from srf_b200 import _lib, ops
 from srf_b200.physics import permuted_sum
 
 COPIES = {"aten::clone", "aten::copy_", "aten::_to_copy"}
@@ -45,6 +45,38 @@ def test_several_views_add_in_order():
     out = permuted_sum(views)
     assert out.is_contiguous() and torch.equal(out, (a + b) + c)
     assert torch.equal(a, views[0])  # sources stay as they were
+
+
+class Cuda:
+    """What ``ops.permutable`` looks at of a CUDA tensor."""
+
+    is_cuda, dtype, requires_grad = True, torch.float32, False
+
+    def __init__(self, *shape, neg=False):
+        self.meta = torch.empty(shape, device="meta")
+        self.shape, self.neg = self.meta.shape, neg
+
+    def dim(self):
+        return self.meta.dim()
+
+    def numel(self):
+        return self.meta.numel()
+
+    def stride(self, k=None):
+        return self.meta.stride() if k is None else self.meta.stride(k)
+
+    def is_neg(self):
+        return self.neg
+
+
+def test_what_the_one_pass_kernel_takes():
+    """Images and stacks that it cannot index, or that are negated on reading, stay with torch."""
+    assert ops.permutable(Cuda(1290, 1290, 1290))
+    assert not ops.permutable(Cuda(1291, 1291, 1291))        # 2^31 voxels and more
+    assert ops.permutable(Cuda(4, 1290, 1290, 1290))
+    assert ops.permutable(Cuda((1 << 31) - 1, 1, 2, 3))
+    assert not ops.permutable(Cuda(1 << 31, 1, 2, 3))        # 2^31 tiles
+    assert not ops.permutable(Cuda(64, 64, 64, neg=True))
 
 
 def _call(dims, frames, strides, sources=(4096,), out=8192):
