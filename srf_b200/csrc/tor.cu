@@ -1634,18 +1634,24 @@ int slab_grid_mult(int op, const SegPlan &sp, int64_t lors_per_launch) {
 }
 
 // Whether the LOR-centric kernels do a call sooner. A slab call costs ~45 us (projection) or
-// ~75 us (scatter) before its first LOR: four or five launches, slabs of 220 KB loaded or
+// ~55 us (scatter) before its first LOR: four or five launches, slabs of 220 KB loaded or
 // cleared and flushed, and a lane walking up to a slab's depth of slices alone. The
-// LOR-centric kernels are one launch and take ~1e-6 us (projection) or 1.7e-6 us (scatter)
-// per LOR, window voxel and slice, so they win up to ~5e7 of those (with every slice of the
-// grid counted: LORs are not longer), four times that where the slabs outnumber the SMs and
-// a CTA goes through several. Measured, slab against LOR-centric, us per projection and
-// back-projection call: 5k LORs at 128 x 128 x 64, patch 6: 111 / 42, 10k 118 / 63 (uncut
-// LORs 141 / 117), 20k 139 / 114 (uncut 175 / 210); 40k at 64 x 64 x 32, patch 4: 143 / 62;
-// 40k at 101 x 93 x 47, patch 3: 157 / 107; 10k at 256 x 256 x 128, patch 7: 962 / 89.
+// LOR-centric kernels are one launch, but a warp takes a LOR 32 slices at a time, however few
+// there are: ~1e-6 us per LOR, window voxel and slice of whole rounds, where the slab kernels
+// take up to half of that for the slices of the grid. So they win up to ~2.5e7 of the
+// difference, 2.5 times that where the slabs outnumber the SMs and a CTA goes through several.
+// Measured, slab against LOR-centric, us per projection / back-projection / both in one call:
+// 128 x 128 x 64, patch 6: 15k LORs 61 / 78 / 112 against 38 / 41 / 77, 30k 70 / 93 / 135
+// against 67 / 71 / 137; 64 x 64 x 32, patch 4: 90k 72 / 88 / 142 against 59 / 61 / 119, 120k
+// 74 / 91 / 146 against 77 / 79 / 153; flat grids: 64 x 64 x 8 60k 38 / 43 / 62 against
+// 40 / 44 / 83, 128 x 128 x 8 40k 48 / 58 / 86 against 46 / 47 / 91, 128 x 128 x 1 1.3M
+// 110 / 118 / 164 against 910 / 1004 / 1918; many slabs: 256 x 256 x 128 (192 slabs) 20k
+// 95 / 141 / 209 against 88 / 115 / 201, 256 frames of 64 x 64 x 8 100k both 135 against 140,
+// 160 frames of 64 x 64 x 32 200k both 341 against 314.
 bool few_lors(const TorParams &p, const SegPlan &sp) {
-    const double work = (double)p.n * p.patch * p.patch * p.gz;
-    return work <= (sp.n_slabs > num_sms() ? 2.0e8 : 5.0e7);
+    const double rounds = 32.0 * ((p.gz + 31) / 32);
+    const double work = (double)p.n * p.patch * p.patch * (rounds - 0.5 * p.gz);
+    return work <= (sp.n_slabs > num_sms() ? 6.25e7 : 2.5e7);
 }
 
 // Events [c0, c0 + n) of p as a call of their own (same images and outputs' layout).
