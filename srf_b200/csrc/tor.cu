@@ -933,10 +933,13 @@ __device__ __forceinline__ SlabIdLor slab_id_lor(const TorParams &p, const SegPl
     // parameter, clamped, then its row, then conversions to integer took twice the
     // instructions: count and fill of 4M events at 256 x 256 x 128 1.10 -> 0.70 ms, of 3M
     // generated pairs there 3.23 -> 2.41 ms.)
-    const float m = d1 / dz * p.inv_y;
+    // The terms of row0 may be far larger than their sum (an image or LORs far from the
+    // origin): 2^-21 of them covers their roundings.
+    const float m = d1 / dz * p.inv_y, up = m * (p.slice0_f - z1), y = y1 * p.inv_y;
     c.drow = m * p.inter_z;
-    c.row0 = fmaf(m, p.slice0_f - z1, fmaf(y1, p.inv_y, p.box_y0));
-    c.reach = fminf(byv, (float)p.patch + 1.0f) + 0.02f + 0.02f * fabsf(c.drow);
+    c.row0 = up + (y + p.box_y0);
+    c.reach = fminf(byv, (float)p.patch + 1.0f) + 0.02f + 0.02f * fabsf(c.drow) +
+              4.77e-7f * (fabsf(up) + fabsf(y) + fabsf(p.box_y0));
     if (!(fabsf(c.row0) < kAllRows && c.reach < kAllRows)) {
         c.row0 = c.drow = 0.0f;  // every band, left to the exact per-slice test
         c.reach = kAllRows;
@@ -1543,6 +1546,12 @@ int tor_setup(TorParams &p, const int *grid, const float *center, const float *s
     p.box_x0 = -p.l_bound * p.inv_x - 0.5f;
     p.box_y0 = -p.b_bound * p.inv_y - 0.5f;
     p.fit = std::min((float)p.half + 0.5f, (float)(p.patch - p.half) - 0.5f) - 1.0f / 1024.0f;
+    // Without a window a box starts at cx / inter_x + box_x0 - bxv, four roundings of a number
+    // of the size of the coordinates in voxels; the half-extents' margin of 1/1024 covers them
+    // up to 4096 voxels from the origin. Images further out always walk the window.
+    if (!(std::max(std::fabs(p.l_bound) * p.inv_x + (float)gx,
+                   std::fabs(p.b_bound) * p.inv_y + (float)gy) < 4096.0f))
+        p.fit = 0.0f;
     auto twice = [](float a) {
         unsigned u;
         std::memcpy(&u, &a, sizeof u);
