@@ -934,12 +934,13 @@ __device__ __forceinline__ SlabIdLor slab_id_lor(const TorParams &p, const SegPl
     // instructions: count and fill of 4M events at 256 x 256 x 128 1.10 -> 0.70 ms, of 3M
     // generated pairs there 3.23 -> 2.41 ms.)
     // The terms of row0 may be far larger than their sum (an image or LORs far from the
-    // origin): 2^-21 of them covers their roundings.
+    // origin): 2^-21 of them covers their roundings, and those of the slices' planes.
     const float m = d1 / dz * p.inv_y, up = m * (p.slice0_f - z1), y = y1 * p.inv_y;
+    const float along = fabsf(m) * (fabsf(p.slice0_f) + fabsf(z1));
     c.drow = m * p.inter_z;
     c.row0 = up + (y + p.box_y0);
     c.reach = fminf(byv, (float)p.patch + 1.0f) + 0.02f + 0.02f * fabsf(c.drow) +
-              4.77e-7f * (fabsf(up) + fabsf(y) + fabsf(p.box_y0));
+              4.77e-7f * (along + fabsf(y) + fabsf(p.box_y0));
     if (!(fabsf(c.row0) < kAllRows && c.reach < kAllRows)) {
         c.row0 = c.drow = 0.0f;  // every band, left to the exact per-slice test
         c.reach = kAllRows;

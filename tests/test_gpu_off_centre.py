@@ -49,3 +49,27 @@ def test_off_centre(grid, path, off):
     assert np.max(np.abs(pv - ref) / np.maximum(np.abs(ref), 1e-3 * ref.max())) <= 1e-5
     ref = O.tor_backprojection(soa, np.ones(n, np.float32), *a, mode="f32", contract=True)
     assert K.rel_l2(bp.cpu().numpy(), ref) <= 1e-5
+
+
+def test_off_centre_along_the_slices():
+    """Planes that lie half a slice from where an even spacing would put them: rows of bands
+    (128 x 128 slices in bands of 25 rows) are still all reached."""
+    grid, n, voxel, kw, off = [128, 128, 26], 40_000, 3.2, 10.19, 1.6e7
+    size = [k * voxel for k in grid]
+    centre = [0.0, 0.0, off]
+    lors = _lors(n, size, centre)
+    img = torch.rand(grid[::-1], device="cuda", generator=torch.Generator("cuda").manual_seed(3))
+    img += 0.1
+    a = (grid, centre, size, kw, False, 6.0, 1.0e6)
+    tuning.set_tuning(1, 16, 0)
+    try:
+        pv = ops.tor_projection(lors, img, *a, layout="nc").cpu().numpy()
+        bp = ops.tor_backprojection(img, lors, torch.ones(n, device="cuda"), *a, layout="nc")
+    finally:
+        tuning.set_tuning()
+    soa = np.ascontiguousarray(lors.cpu().numpy().T)
+    ref = O.tor_projection(soa, img.cpu().numpy(), *a, mode="f32", contract=True)
+    assert np.count_nonzero(ref) > 0.9 * n
+    assert np.max(np.abs(pv - ref) / np.maximum(np.abs(ref), 1e-3 * ref.max())) <= 1e-5
+    ref = O.tor_backprojection(soa, np.ones(n, np.float32), *a, mode="f32", contract=True)
+    assert K.rel_l2(bp.cpu().numpy(), ref) <= 1e-5
