@@ -688,7 +688,8 @@ __device__ __forceinline__ bool seg_value(const TorParams &p, int64_t t, SegLor 
     if (!lor_value_scale<OP>(p, t, c)) return false;
     L.scale = c.scale;
     L.general = L.general || c.all || !(fabsf(c.scale) <= 3.0e38f);
-    if (OP != kProj && c.scale == 0.0f) return L.general;  // finite weights times 0
+    // 0 times the weights: they are finite unless they grow towards the cut-off
+    if (OP != kProj && c.scale == 0.0f && !(L.k1 > 0.0f)) return L.general;
     if (OP == kBack) L.kE += c.k0s;
     return true;
 }
@@ -1318,9 +1319,9 @@ __device__ __forceinline__ float walk_segment(const TorParams &p, const SlabView
     return acc0 + acc1;
 }
 
-// A segment whose LOR takes the general walk (a map LOR with a zero or non-finite divisor,
-// a LOR far from the slice axis or with a TOF centre that is not finite): its slices [S0, S1) and rows [R0, R1) straight on the
-// image in global memory.
+// A segment whose LOR takes the general walk (a map LOR with a zero or non-finite divisor, a
+// LOR far from the slice axis or with a TOF centre that is not finite): its slices [S0, S1)
+// and rows [R0, R1) straight on the image in global memory.
 template <int OP, int P>
 __device__ __noinline__ void general_segment(const TorParams &p, int64_t t, int S0, int S1,
                                              int R0, int R1, int64_t img0) {

@@ -160,3 +160,25 @@ def test_centre_at_infinity(row, value):
     for got in (ops.tor_backprojection(img, L, V, *a, layout="cn"),
                 ops.tor_backproject_adjoint(0.25 * V, L, *a, layout="cn")):
         assert K.rel_l2(got.cpu().numpy(), ref) <= 1e-5
+
+
+def test_zero_values_and_weights_beyond_the_floats():
+    """TOF so sharp that weights overflow towards the cut-off (e^220): a zero value leaves
+    infinity times 0 there, not a number, as in the LOR-centric kernels, and 0 elsewhere."""
+    n, voxel, kw, tof = 20, 6.4, 24.0, (0.5, 0.3)
+    size = [g * voxel for g in GRID]
+    lors = _lors(n, 17)
+    at = np.arange(n)  # along z, centres in slice planes
+    lors[0, at] = lors[3, at] = lors[6, at] = (at - 10) * 9.7
+    lors[1, at] = lors[4, at] = lors[7, at] = (at % 5 - 2) * 11.3
+    lors[2, at], lors[5, at], lors[8, at] = -300.0, 300.0, (at % 9 - 4 + 0.5) * voxel
+    lors[9, at] = 1.0
+    L, V = _cu(lors), torch.zeros(n, device="cuda")
+    a = (GRID, CENTER, size, kw, False, *tof)
+    got = ops.tor_backproject_adjoint(V, L, *a, layout="cn")
+    tuning.set_tuning(2, 0, 0)
+    ref = ops.tor_backproject_adjoint(V, L, *a, layout="cn")
+    nan = torch.isnan(ref)
+    assert nan.any() and not nan.all()
+    assert torch.equal(torch.isnan(got), nan)
+    assert not got[~nan].any() and not ref[~nan].any()
