@@ -17,10 +17,10 @@ from tests import _cases as K
 pytestmark = pytest.mark.gpu
 
 
-def _lors(n, size, centre):
+def _lors(n, size, centre, slope=0.6):
     g = np.random.default_rng(5)
     mid = (g.random((n, 3)) - 0.5) * np.array(size) * 0.9 + np.array(centre)
-    d = np.stack([g.uniform(-0.6, 0.6, n), g.uniform(-0.6, 0.6, n), np.ones(n)], 1)
+    d = np.stack([g.uniform(-slope, slope, n), g.uniform(-slope, slope, n), np.ones(n)], 1)
     d /= np.linalg.norm(d, axis=1, keepdims=True)
     rec = np.concatenate([mid - 300 * d, mid + 300 * d, mid, np.ones((n, 1))], 1)
     return torch.as_tensor(rec.astype(np.float32)).cuda()
@@ -52,12 +52,13 @@ def test_off_centre(grid, path, off):
 
 
 def test_off_centre_along_the_slices():
-    """Planes that lie half a slice from where an even spacing would put them: rows of bands
-    (128 x 128 slices in bands of 25 rows) are still all reached."""
-    grid, n, voxel, kw, off = [128, 128, 26], 40_000, 3.2, 10.19, 1.6e7
+    """Planes that lie up to half a millimetre from where an even spacing would put them (floats
+    are 1 mm apart there): every row of every band (128 x 128 slices, 16 per slab) that oblique
+    LORs reach still has them."""
+    grid, n, voxel, kw, off = [128, 128, 26], 40_000, 2.7, 10.19, 1.6e7
     size = [k * voxel for k in grid]
     centre = [0.0, 0.0, off]
-    lors = _lors(n, size, centre)
+    lors = _lors(n, size, centre, slope=1.5)
     img = torch.rand(grid[::-1], device="cuda", generator=torch.Generator("cuda").manual_seed(3))
     img += 0.1
     a = (grid, centre, size, kw, False, 6.0, 1.0e6)
