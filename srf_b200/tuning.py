@@ -45,7 +45,7 @@ def candidates(max_slab_slices):
     """Settings worth trying: full and half-depth slabs, each with the library's automatic
     grid multiplier (0: chosen per op and call size) and with multipliers 1 and 2 fixed,
     path 3 (the slab kernels again, kept for stored settings) and the LOR-centric kernels.
-    The automatic choice comes first, so a tie keeps it."""
+    The slab kernels' automatic settings come first, so a tie keeps them."""
     out = [(1, 0, 0), (1, 0, 1), (1, 0, 2)]
     half = max(1, max_slab_slices // 2)
     if half < max_slab_slices:
